@@ -20,6 +20,7 @@
 // TMEM is released.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -28,6 +29,9 @@
 
 #include "internal.h"
 #include "requant.h"
+#include "tc_common.cuh"
+#include "tc_host.h"
+#include "gconv.cuh"
 
 namespace enn_b200 {
 
@@ -52,9 +56,6 @@ namespace {
 #define ENN_DBG_PTR(p) static_cast<long long *>(nullptr)
 #endif
 
-constexpr int kBM = 128;            // rows per tile = UMMA M
-constexpr int kBK = 128;            // bytes of K per stage = one 128B swizzle atom = 4 UMMA K steps
-constexpr int kMaxBN = 256;         // UMMA N limit
 // Epilogue warps: 3 per TMEM lane quarter, splitting the 16-column chunks.  The epilogue is bound by dependent integer
 // latencies, not by warp count: 12 warps with 128 registers (room for the compiler to interleave the 8 outputs of a half
 // chunk) run the MobileNetV2 graph 6 % faster than 24 warps capped at 72 registers; 8 and 16 warps are 1 % behind.
@@ -68,14 +69,7 @@ constexpr int kChunksPerWarp = (kMaxBN / 16 + kColGroups - 1) / kColGroups;   //
 // over 100 registers itself, and with 80 / 144 the 1x1 layers ran 40 % slower.)
 constexpr int kThreadsOneProducer = 64 + 32 * kEpiWarps;
 constexpr int kThreads = kThreadsOneProducer + 32;
-constexpr uint32_t kSpinLimit = 1u << 24;
-
-struct ColParam {   // per output column, 16 bytes
-    int32_t mult;
-    int32_t addend;   // stage-2 addend: 2^(e-1) + ((out_zp - act_min) << e)
-    int32_t esh;      // right shift e >= 1 of the fused form; negative: general requantisation, `addend` = raw shift
-    int32_t bias;     // folded bias'
-};
+constexpr size_t kWidePackWeightBytes = 100 * 1024;    // resident block-diagonal weights of a wide-row pixel packing
 
 struct TcParams {
     int32_t M, N, K;
@@ -125,211 +119,6 @@ struct TcParams {
     int32_t test_starve;    // self-test of the bounded waits: no operand copy is issued and the waits give up early
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait of the single-thread roles (producers, MMA issuer).  Callers look at the barrier with the non-blocking
-// test_wait first (the common case: already complete); what is left waits with try_wait, which parks the thread in
-// hardware between looks instead of spinning through issue slots that the epilogue warps of the same scheduler need.
-__device__ __forceinline__ bool mbar_wait_fast(uint32_t bar, uint32_t parity, volatile int *abort_flag, int32_t *err, int code,
-                                               uint32_t looks = kSpinLimit >> 7) {
-    for (uint32_t i = 0; i < looks; ++i) {       // by default 2^17 looks of up to 10 us: gives up after about a second
-        // suspend-time hint (ns): stay parked until the phase completes instead of coming back every few hundred cycles
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity), "r"(10000u)
-            : "memory");
-        if (ok) return true;
-        if ((i & 63u) == 63u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    if (err) *reinterpret_cast<volatile int32_t *>(err) = code;
-    return false;
-}
-// Bounded wait.  Returns false after the limit (or when another thread already aborted the CTA).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int32_t *err, int code) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    if (err) *reinterpret_cast<volatile int32_t *>(err) = code;
-    return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t c0, int32_t c1) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Arrives on the mbarrier once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// ---- CTA-pair (cta_group::2) forms: two CTAs of a cluster compute one 256-row tile, each holding its own 128 rows of
-// A, half of the B rows and its 128 accumulator lanes.  The MMA is issued by the rank-0 CTA only.
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Address of the same shared-memory offset in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t mapa_rank(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The tile lands in this CTA's shared memory; the bytes are counted on the rank-0 CTA's barrier (cluster address).
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar_cluster, int32_t c0, int32_t c1) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t slot_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-// Arrives on the barrier at this offset in both CTAs of the pair once the MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    const uint16_t mask = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask) : "memory");
-}
-
-// One k-block: KS (1, 2 or 4) MMAs over consecutive 32-byte K slices of the A tile at descriptor address `lo_a` and the
-// B tile at `lo_b` (16-byte units; `desc_hi` = the constant upper descriptor word).  All descriptors are formed first, then
-// the MMAs follow each other as one uninterrupted instruction run.  The first MMA overwrites the accumulator when
-// `accumulate_first` is 0.
-template <bool TWO, int KS>
-__device__ __forceinline__ void umma_i8_run(uint32_t d_tmem, uint32_t desc_hi, uint32_t lo_a, uint32_t lo_b, uint32_t idesc,
-                                            uint32_t accumulate_first) {
-#define ENN_MMA_PAIR "tcgen05.mma.cta_group::2.kind::i8"
-#define ENN_MMA_ONE "tcgen05.mma.cta_group::1.kind::i8"
-#define ENN_DESC(I, OFF)                                                       \
-    "add.u32 t, %2, " #OFF ";\n\tmov.b64 a" #I ", {t, %1};\n\t"                 \
-    "add.u32 t, %3, " #OFF ";\n\tmov.b64 b" #I ", {t, %1};\n\t"
-#define ENN_RUN_HEAD                                                                                  \
-    "{\n\t.reg .pred p, q;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t.reg .b32 t;\n\t"           \
-    "setp.ne.b32 p, %5, 0;\n\t"                                                                       \
-    "setp.eq.b32 q, %5, %5;\n\t"
-#define ENN_RUN_ARGS ::"r"(d_tmem), "r"(desc_hi), "r"(lo_a), "r"(lo_b), "r"(idesc), "r"(accumulate_first) : "memory"
-#define ENN_RUN(MMA)                                                                                                   \
-    if (KS == 4)                                                                                                       \
-        asm volatile(ENN_RUN_HEAD ENN_DESC(0, 0) ENN_DESC(1, 2) ENN_DESC(2, 4) ENN_DESC(3, 6)                         \
-                     MMA " [%0], a0, b0, %4, p;\n\t" MMA " [%0], a1, b1, %4, q;\n\t" MMA " [%0], a2, b2, %4, q;\n\t" \
-                     MMA " [%0], a3, b3, %4, q;\n\t}" ENN_RUN_ARGS);                                                   \
-    else if (KS == 2)                                                                                                  \
-        asm volatile(ENN_RUN_HEAD ENN_DESC(0, 0) ENN_DESC(1, 2)                                                       \
-                     MMA " [%0], a0, b0, %4, p;\n\t" MMA " [%0], a1, b1, %4, q;\n\t}" ENN_RUN_ARGS);                   \
-    else                                                                                                               \
-        asm volatile(ENN_RUN_HEAD ENN_DESC(0, 0) MMA " [%0], a0, b0, %4, p;\n\t}" ENN_RUN_ARGS);
-    if (TWO) { ENN_RUN(ENN_MMA_PAIR) } else { ENN_RUN(ENN_MMA_ONE) }
-#undef ENN_RUN
-#undef ENN_RUN_ARGS
-#undef ENN_RUN_HEAD
-#undef ENN_DESC
-#undef ENN_MMA_ONE
-#undef ENN_MMA_PAIR
-}
-
-__device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_x1(uint32_t taddr, uint32_t &r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// K-major operand tile in shared memory, 128-byte rows, 128B swizzle: rows are 128 bytes apart, groups of 8
-// rows 1024 bytes apart (stride byte offset), descriptor version 1, layout type 2 (SWIZZLE_128B).
-// `span` = bytes per row = swizzle span (128 / 64 / 32): groups of 8 rows are 8 * span bytes apart and the layout
-// type is SWIZZLE_128B (2), SWIZZLE_64B (4) or SWIZZLE_32B (6).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t span = 128) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);        // start address, 16-byte units
-    d |= static_cast<uint64_t>(1) << 16;                            // leading byte offset (unused for swizzled K-major)
-    d |= static_cast<uint64_t>((8 * span) >> 4) << 32;              // stride byte offset
-    d |= static_cast<uint64_t>(1) << 46;                            // descriptor version
-    d |= static_cast<uint64_t>(span == 128 ? 2 : (span == 64 ? 4 : 6)) << 61;
-    return d;
-}
-
-__device__ __forceinline__ uint32_t pack_sat_u8_tc(int32_t hi, int32_t lo, uint32_t upper) {
-    uint32_t d;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
-    return d;
-}
-
 // Work unit `tile` -> (M tile group tg, N tile tn).  Units are numbered band by band: a band is `raster` consecutive M
 // groups, and inside a band the M index runs fastest.  The units in flight at one time (one per SM) then share few A and
 // few B tiles, so that both operands stay L2 resident for large problems.
@@ -354,86 +143,6 @@ __device__ __forceinline__ void tile_coords(const TcParams &p, int tile, int &tg
     const int gw = min(p.raster, p.tiles_mg - g0);      // the last band may be narrower
     tn = r / gw;
     tg = g0 + (r - tn * gw);
-}
-
-// Epilogue modes (one kernel variant each; the planner picks the cheapest one every column of the operator allows):
-//   kModeNudge   fused two-stage form below, every column a right shift e >= 1;
-//   kModeGeneral as kModeNudge, but columns flagged esh < 0 take the general code (left shifts, e == 0, wide ranges);
-//   kModeReluTwo lower clamp == output zero point (ReLU-type outputs): a negative stage-1 value ends at the clamp with or
-//                without the tie correction, so the correction is dropped and the bias, both rounding terms and a left
-//                shift ls fold into one 64-bit addend: q = acc * M0 + C, C = bias * M0 + 2^(30-ls) (+ 2^(e-1+31-ls) when
-//                e >= 1); result = (q >> (31 - ls)) >> e.  Covers e == 0 and left shifts, which otherwise need the
-//                general code.
-//   kModeReluHi  the same with one shift, hi32(q) >> (e - 1), for operators whose columns all have e >= 1 and ls == 0
-//                (two ALU instructions per output fewer; option no_relu_hi keeps the two-shift form).
-// ColParam words: {mult, addend, esh, bias} for the first two modes, {C low, C high, mult, shifts} for the ReLU modes
-// (shifts = e - 1 for kModeReluHi, (31 - ls) | e << 8 for kModeReluTwo).
-constexpr size_t kWidePackWeightBytes = 100 * 1024;    // resident block-diagonal weights of a wide-row pixel packing
-constexpr int kModeNudge = 0, kModeGeneral = 1, kModeReluHi = 2, kModeReluTwo = 3;
-// kModeReluHi for outputs whose clamp is the whole unsigned byte (lower clamp 0, upper clamp 255, unsigned bytes): the
-// saturating byte pack is the clamp, so the min / max and the add of the lower clamp to the packed word are left out.
-// A kernel template value only: the plan and the ColParam contents are those of kModeReluHi.
-constexpr int kModeReluSat = 4;
-
-// The constants of one column in registers.  The ReLU modes read {C, (M0, shifts)} as two 64-bit words, so that the
-// 64-bit addend arrives as a register pair and need not be assembled from two 32-bit registers.
-struct ColRegs {
-    int4 v;
-    int64_t cc;
-};
-// `p` points into shared memory (derived from the kernel's shared array, so the compiler emits shared loads with
-// the constant part of the address as the instruction's immediate offset).
-template <int MODE>
-__device__ __forceinline__ void ld_col_shared(const uint8_t *p, ColRegs &c) {
-    __builtin_assume(__isShared(p));
-    if (MODE >= kModeReluHi) {
-        const longlong2 v = *reinterpret_cast<const longlong2 *>(p);
-        c.cc = v.x;
-        asm("mov.b64 {%0, %1}, %2;" : "=r"(c.v.z), "=r"(c.v.w) : "l"(v.y));
-    } else {
-        c.v = *reinterpret_cast<const int4 *>(p);
-    }
-}
-
-// Requantise one accumulator (bias not yet added) to (value - act_min) in [0, act_max - act_min]; kModeReluSat leaves
-// the clamp to the caller's saturating pack.
-// Fast form (esh = right shift e >= 1): stage 1 is one 32x32->64 multiply-add and a funnel shift, stage 2 is
-// (x + addend - [x < 0]) >> e with addend = 2^(e-1) + ((out_zp - act_min) << e), i.e. RoundingDivideByPOT
-// (ties away from zero) with the zero point and the lower clamp folded in.
-template <int MODE>
-__device__ __forceinline__ int32_t tc_requant(int32_t acc, const ColRegs &cr, int32_t hi_clamp, int32_t out_zp, int32_t act_min,
-                                              int32_t act_max) {
-    const int4 &c = cr.v;
-    if (MODE >= kModeReluHi) {
-        const int64_t q = static_cast<int64_t>(acc) * c.z + cr.cc;
-        int32_t lo, hi;
-        asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(q));
-        int32_t v;
-        if (MODE == kModeReluTwo) {
-            const int32_t xa = static_cast<int32_t>(__funnelshift_r(static_cast<uint32_t>(lo), static_cast<uint32_t>(hi), static_cast<uint32_t>(c.w)));
-            v = xa >> (c.w >> 8);
-        } else {
-            v = hi >> c.w;
-        }
-        if (MODE == kModeReluSat) return v;
-        return __vimin_s32_relu(v, hi_clamp);
-    }
-    acc += c.w;
-    if (MODE == kModeGeneral && c.z < 0) return enn_requant(acc, c.x, c.y, out_zp, act_min, act_max) - act_min;   // c.y = raw shift
-    const int64_t p = static_cast<int64_t>(acc) * c.x + (1ll << 30);
-    const int32_t x = static_cast<int32_t>(p >> 31);
-    const int32_t v = (x + c.y - static_cast<int32_t>(static_cast<uint32_t>(x) >> 31)) >> c.z;
-    return __vimin_s32_relu(v, hi_clamp);
-}
-// The same from the four 32-bit words of a ColParam.
-template <int MODE>
-__device__ __forceinline__ int32_t tc_requant(int32_t acc, const int4 &c, int32_t hi_clamp, int32_t out_zp, int32_t act_min,
-                                              int32_t act_max) {
-    ColRegs cr;
-    cr.v = c;
-    cr.cc = 0;
-    if (MODE >= kModeReluHi) asm("mov.b64 %0, {%1, %2};" : "=l"(cr.cc) : "r"(c.x), "r"(c.y));
-    return tc_requant<MODE>(acc, cr, hi_clamp, out_zp, act_min, act_max);
 }
 
 // The k loop of one accumulator tile for the common big-GEMM shape (four K slices per k-block, one k-block per stage),
@@ -475,38 +184,6 @@ ENN_TILE_FN(mma_tile_d4, 4, case 0: ENN_KB(0) case 1: ENN_KB(1) case 2: ENN_KB(2
 ENN_TILE_FN(mma_tile_d6, 6, case 0: ENN_KB(0) case 1: ENN_KB(1) case 2: ENN_KB(2) case 3: ENN_KB(3) case 4: ENN_KB(4) case 5: ENN_KB(5))
 #undef ENN_TILE_FN
 #undef ENN_KB
-
-// Fused add: the 16 requantised bytes of a chunk (four words) and the 16 bytes of the other addend at the same place go
-// through the quantized add exactly as add_kernel_vec computes it (kernels_direct.cu): stage 1 of either input from the
-// operator's tables in shared memory, stage 2 computed.
-struct FaddCtx {
-    uint32_t lut_u32;       // 2 x 256 words in shared memory: input-0 table, input-1 table
-    int32_t mo, so, out_off, act_min, act_max;
-    bool swap;
-};
-__device__ __forceinline__ uint32_t fadd_word(uint32_t y, uint32_t r, const FaddCtx &f) {
-    const uint32_t a = f.swap ? r : y, b = f.swap ? y : r;
-    uint32_t word = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t ba = (a >> (8 * k)) & 0xff, bb = (b >> (8 * k)) & 0xff;
-        int32_t x0, x1;
-        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x0) : "r"(f.lut_u32 + ba * 4));
-        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x1) : "r"(f.lut_u32 + 1024 + bb * 4));
-        int32_t o = enn_rdivpot(enn_srdhm(x0 + x1, f.mo), -f.so) + f.out_off;
-        o = max(f.act_min, o);
-        o = min(f.act_max, o);
-        word |= (static_cast<uint32_t>(o) & 0xff) << (8 * k);
-    }
-    return word;
-}
-__device__ __forceinline__ void fadd_chunk(uint32_t (&w)[4], const uint8_t *res, const FaddCtx &f) {
-    const uint4 r = *reinterpret_cast<const uint4 *>(res);      // plain load: the output may be written over this addend
-    w[0] = fadd_word(w[0], r.x, f);
-    w[1] = fadd_word(w[1], r.y, f);
-    w[2] = fadd_word(w[2], r.z, f);
-    w[3] = fadd_word(w[3], r.w, f);
-}
 
 // TWO: CTA-pair mode (launched as clusters of 2; plain GEMM operands only, group == 1, kpack == 1): the pair owns M
 // tiles 2t and 2t + 1 of one N tile, every B byte is read from L2 once per pair, and a stage per CTA is A plus half of B.
@@ -1581,10 +1258,6 @@ __global__ void __launch_bounds__(256) conv3x3c3_kernel(Conv3x3c3Params g, const
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // One GEMM launch: an operator is one of these (convolution, FullyConnected) or one per output parity class
 // (transposed convolution).
 struct TcGemm {
@@ -1621,6 +1294,7 @@ struct TcPlan {
     std::vector<TcGemm> gemms;
     void *scratch = nullptr;           // im2col matrix, shared by the GEMMs of the op (they run in stream order)
     size_t scratch_bytes = 0;
+    std::unique_ptr<GcPlan> gc;        // gather convolution (gconv.cu): replaces the list of GEMMs
     bool fan_out = false;              // the GEMMs are independent (deconvolution classes): run them side by side
     int32_t *err_host = nullptr;       // pinned + mapped
     int32_t *err_dev = nullptr;
@@ -1628,24 +1302,6 @@ struct TcPlan {
     bool fused_add = false;            // convolution + quantized add (tc_fuse_add)
     const uint8_t *residual = nullptr; // the add's other input for the next execute
 };
-
-CUtensorMapSwizzle swizzle_of(uint32_t span) {
-    return span == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (span == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-}
-
-bool encode_2d(enn_b200_context *ctx, CUtensorMap *map, const void *base, uint64_t inner, uint64_t outer, uint64_t pitch,
-               uint32_t box_inner, uint32_t box_outer) {
-    EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled);
-    if (!fn) return false;
-    cuuint64_t dims[2] = {inner, outer};
-    cuuint64_t strides[1] = {pitch};
-    cuuint32_t box[2] = {box_inner, box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_of(box_inner), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
 
 // NHWC activation tensor {C, W, H, N} with a box of {span channels, box_w, box_h, 1}.
 bool encode_nhwc(enn_b200_context *ctx, CUtensorMap *map, const void *base, uint64_t c, uint64_t w, uint64_t h, uint64_t n, uint32_t span,
@@ -1660,10 +1316,6 @@ bool encode_nhwc(enn_b200_context *ctx, CUtensorMap *map, const void *base, uint
                     swizzle_of(span), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
-
-struct QuantHost {   // host copies of what setup_quant uploaded
-    std::vector<int32_t> mult, shift, bias;
-};
 
 // Builds one GEMM: packs B, folds zero points into the bias, derives the epilogue constants, sizes the launch.
 // weight(n, k) returns the raw weight byte of output column n at reduction index k (k < K).
@@ -1758,9 +1410,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     std::vector<int8_t> wb(static_cast<size_t>(tiles_n) * p.bn_rows * k_pad, 0);
     std::vector<ColParam> cols(static_cast<size_t>(tiles_n) * p.bn_rows);
     std::memset(cols.data(), 0, cols.size() * sizeof(ColParam));
-    const int64_t amax = g.a_signed ? 128 : 255;
-    const int64_t zo_eff = static_cast<int64_t>(g.out_zp) - g.act_min;
-    std::vector<int64_t> folded_v(N), bound_v(N);
+    std::vector<ColumnFold> folds(N);
     for (int32_t n = 0; n < N; ++n) {
         const int32_t tn = n / bn_data, r = n % bn_data;
         int8_t *dst = wb.data() + (static_cast<size_t>(tn) * p.bn_rows + r) * k_pad;
@@ -1772,63 +1422,12 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
             wsum += wv;
             wabs += wv < 0 ? -wv : wv;
         }
-        const int64_t folded = static_cast<int64_t>(qh.bias[n]) - static_cast<int64_t>(g.in_zp) * wsum +
-                               static_cast<int64_t>(K) * g.in_zp * zw_eff;
-        folded_v[n] = folded;
-        // bound on |accumulator + folded bias|
-        bound_v[n] = amax * wabs + static_cast<int64_t>(K) * amax * (zw_eff < 0 ? -zw_eff : zw_eff) + (folded < 0 ? -folded : folded);
+        folds[n] = fold_column(g, qh.bias[n], K, wsum, wabs, zw_eff);
     }
-    // ReLU-type outputs (lower clamp == output zero point): can every column use the merged form?
-    bool relu_hi = zo_eff == 0 && M > kGemvMaxM && !ctx->opt("no_relu_mode"), relu_two = relu_hi;
-    for (int32_t n = 0; n < N && relu_two; ++n) {
-        const int32_t sh = qh.shift[n];
-        const int32_t ls = sh > 0 ? sh : 0, e = sh > 0 ? 0 : -sh;
-        const bool in_range = folded_v[n] <= INT32_MAX && folded_v[n] >= INT32_MIN && bound_v[n] < (1ll << 31) && qh.mult[n] >= 0;
-        if (!in_range || ls > 30 || e > 31) relu_hi = relu_two = false;
-        if (ls > 0 || e < 1) relu_hi = false;
-        // two-shift form: the left-shifted accumulator must not wrap (the reference multiplies in int32) and the
-        // stage-1 value plus the rounding term must fit 32 bits
-        if ((bound_v[n] << ls) + (e >= 1 ? (1ll << (e - 1)) : 0) + 1 >= (1ll << 31)) relu_two = false;
-    }
-    p.mode = relu_hi && !ctx->opt("no_relu_hi") ? kModeReluHi : (relu_two ? kModeReluTwo : kModeNudge);
-    // The clamp is the whole unsigned byte: the saturating pack of the epilogue does it (kModeReluSat).
-    p.sat_plain = p.mode == kModeReluHi && !p.a_signed && p.act_min == 0 && p.act_max >= 255 && !ctx->opt("no_relu_sat");
-    for (int32_t n = 0; n < N; ++n) {
-        const int32_t tn = n / bn_data, r = n % bn_data;
-        const int64_t folded = folded_v[n];
-        ColParam &c = cols[static_cast<size_t>(tn) * p.bn_rows + r];
-        if (p.mode == kModeReluHi || p.mode == kModeReluTwo) {
-            const int32_t sh = qh.shift[n];
-            const int32_t ls = sh > 0 ? sh : 0, e = sh > 0 ? 0 : -sh;
-            int64_t cc = folded * qh.mult[n];
-            int32_t word;
-            if (p.mode == kModeReluHi) {
-                cc += (1ll << 30) + (1ll << (30 + e));
-                word = e - 1;
-            } else {
-                const int32_t s1 = 31 - ls;
-                cc += (1ll << (30 - ls)) + (e >= 1 ? (1ll << (e - 1 + s1)) : 0);
-                word = s1 | (e << 8);
-            }
-            c.mult = static_cast<int32_t>(static_cast<uint32_t>(static_cast<uint64_t>(cc) & 0xffffffffu));   // word 0: C low
-            c.addend = static_cast<int32_t>(static_cast<uint32_t>(static_cast<uint64_t>(cc) >> 32));            // word 1: C high
-            c.esh = qh.mult[n];                                                                                // word 2: M0
-            c.bias = word;                                                                                     // word 3: shifts
-            continue;
-        }
-        c.mult = qh.mult[n];
-        c.bias = static_cast<int32_t>(folded);     // wraps like the reference's int32 accumulation
-        const int32_t e = qh.shift[n] > 0 ? -1 : -qh.shift[n];
-        const int64_t addend = e > 0 ? (1ll << (e - 1)) + zo_eff * (1ll << e) : zo_eff;
-        if (e < 1 || folded > INT32_MAX || folded < INT32_MIN || bound_v[n] + 2 + (addend < 0 ? -addend : addend) >= (1ll << 31)) {
-            c.addend = qh.shift[n];                // general path keeps the raw signed shift
-            c.esh = INT32_MIN;
-            p.mode = kModeGeneral;
-        } else {
-            c.addend = static_cast<int32_t>(addend);
-            c.esh = e;
-        }
-    }
+    p.mode = column_mode(ctx, g, qh, folds, N, M > kGemvMaxM);
+    p.sat_plain = column_sat_plain(ctx, g, p.mode);
+    for (int32_t n = 0; n < N; ++n)
+        if (!column_constants(g, p.mode, qh.mult[n], qh.shift[n], folds[n], &cols[static_cast<size_t>(n / bn_data) * p.bn_rows + n % bn_data])) p.mode = kModeGeneral;
     if (p.need_asum)
         for (int32_t tn = 0; tn < tiles_n; ++tn) {
             int8_t *dst = wb.data() + (static_cast<size_t>(tn) * p.bn_rows + bn_data) * k_pad;
@@ -1879,12 +1478,158 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     return ENN_B200_SUCCESS;
 }
 
+// Plans a gather convolution (gconv.cu) over `classes`; weight(class, n, k) returns the raw weight byte of output column n at
+// reduction index k = (ky * kw + kx) * cin + c of that class.  INVALID_PARAMS: outside what the kernel covers.
+template <typename WeightFn>
+int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh, const std::vector<GcClassDesc> &classes, int32_t sy, int32_t sx,
+                    int64_t out_sn, int64_t out_sy, int64_t out_sx, WeightFn weight, GcPlan *gc) {
+    const int32_t N = g.cout, cin = g.cin, nc = static_cast<int32_t>(classes.size());
+    if (nc < 1 || nc > kGcMaxClasses || (cin & 3) != 0) return ENN_B200_INVALID_PARAMS;
+    if (static_cast<int64_t>(g.n) * g.h * g.w * cin >= (1ll << 31) - (1 << 20)) return ENN_B200_INVALID_PARAMS;      // 32-bit byte offsets
+    GcParams &p = gc->prm;
+    p.n_classes = nc;
+    p.N = N;
+    p.gran = (cin & 15) == 0 ? 16 : ((cin & 7) == 0 ? 8 : 4);
+    p.h = g.h; p.w = g.w; p.cin = cin; p.sy = sy; p.sx = sx;
+    p.out_sn = out_sn; p.out_sy = out_sy; p.out_sx = out_sx;
+    p.zw_eff = g.w_signed ? g.w_zp : g.w_zp - 128;
+    p.need_asum = p.zw_eff != 0;
+    p.a_signed = g.a_signed;
+    p.act_min = g.act_min; p.act_max = g.act_max; p.out_zp = g.out_zp;
+    const int32_t extra = p.need_asum ? 16 : 0, max_data = kMaxBN - extra;
+    const int sms = ctx->launch_sms();
+    int64_t tiles_m = 0;
+    int32_t k_pad = 0, kb_total = 0;
+    for (int32_t i = 0; i < nc; ++i) {
+        const GcClassDesc &d = classes[i];
+        const int64_t M = static_cast<int64_t>(g.n) * d.oh * d.ow, K = static_cast<int64_t>(d.kh) * d.kw * cin;
+        if (M <= 0 || M > INT32_MAX - kBM || K > (1 << 20)) return ENN_B200_INVALID_PARAMS;
+        if ((d.kh - 1) * std::abs(d.dy) >= 32000 || (d.kw - 1) * std::abs(d.dx) >= 32000 || g.h >= 32000 || g.w >= 32000) return ENN_B200_INVALID_PARAMS;
+        GcClass &c = p.cls[i];
+        c.M = static_cast<int32_t>(M);
+        c.tiles_m = static_cast<int32_t>((M + kBM - 1) / kBM);
+        c.k_blocks = static_cast<int32_t>((K + kBK - 1) / kBK);
+        const int32_t real = static_cast<int32_t>((K - static_cast<int64_t>(c.k_blocks - 1) * kBK + 31) >> 5);
+        c.ks_last = real <= 1 ? 1 : (real == 2 ? 2 : 4);
+        c.oh = d.oh; c.ow = d.ow; c.y0 = d.y0; c.x0 = d.x0;
+        c.div_ow = FastDiv::make(static_cast<uint32_t>(d.ow));
+        c.div_img = FastDiv::make(static_cast<uint32_t>(d.oh) * static_cast<uint32_t>(d.ow));
+        c.out_base = d.out_base;
+        c.tab0 = kb_total * (kBK / p.gran);
+        tiles_m += c.tiles_m;
+        kb_total += c.k_blocks;
+        k_pad = std::max(k_pad, c.k_blocks * kBK);
+    }
+    p.tab_entries = kb_total * (kBK / p.gran);
+    if (p.tab_entries > 3072) return ENN_B200_INVALID_PARAMS;       // 24 KB of gather table
+    // N tiling: as few tiles as possible (every N tile gathers the A tile again), but split while SMs would idle.
+    int32_t tiles_n = (N + max_data - 1) / max_data;
+    while (tiles_m * tiles_n < sms && (N + tiles_n) / (tiles_n + 1) >= 32) ++tiles_n;
+    p.bn_data = (((N + tiles_n - 1) / tiles_n) + 15) & ~15;
+    p.tiles_n = tiles_n = (N + p.bn_data - 1) / p.bn_data;
+    p.bn_rows = p.bn_data + extra;
+    if (tiles_m * tiles_n > INT32_MAX / 2) return ENN_B200_INVALID_PARAMS;
+    int32_t unit = 0, b_tile = 0;
+    for (int32_t i = 0; i < nc; ++i) {
+        p.cls[i].unit0 = unit;
+        p.cls[i].b_tile0 = b_tile;
+        unit += p.cls[i].tiles_m * tiles_n;
+        b_tile += tiles_n * p.cls[i].k_blocks;
+    }
+    p.n_units = unit;
+    p.n_acc = 2 * p.bn_rows <= kMaxBN ? 2 : 1;
+    p.tmem_cols = 32;
+    while (p.tmem_cols < p.n_acc * p.bn_rows) p.tmem_cols *= 2;
+    p.idesc = (2u << 4) | (static_cast<uint32_t>(g.a_signed ? 1 : 0) << 7) | (1u << 10) | (static_cast<uint32_t>(p.bn_rows >> 3) << 17) |
+              (static_cast<uint32_t>(kBM >> 4) << 24);
+    p.b_bytes = p.bn_rows * kBK;
+    p.cols_all = nc * tiles_n * p.bn_rows <= 1024;      // 16 KB
+    // Weights stay in shared memory where three stages of A fit beside them, else they travel with the stages.
+    const uint32_t b_total = static_cast<uint32_t>(std::min<int64_t>(static_cast<int64_t>(b_tile) * p.b_bytes, 1 << 20));
+    p.b_res = 1;
+    p.stages = 3;
+    if (b_total > 64 * 1024 || gconv_smem_bytes(p, b_total) > kGcSmemLimit) p.b_res = 0;
+    p.stages = 4;
+    while (p.stages > 2 && gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) --p.stages;
+    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
+    gc->smem_bytes = gconv_smem_bytes(p, p.b_res ? b_total : 0);
+    gc->grid = p.n_units < 2 * sms ? p.n_units : 2 * sms;
+
+    std::vector<int8_t> wb(static_cast<size_t>(nc) * tiles_n * p.bn_rows * k_pad, 0);
+    std::vector<ColumnFold> folds(static_cast<size_t>(nc) * N);
+    // gather table, then 16 bytes of the input zero point
+    const int fill = static_cast<int>((static_cast<uint32_t>(g.in_zp) & 0xff) * 0x01010101u);
+    const size_t fill_at = static_cast<size_t>(p.tab_entries + 1) & ~static_cast<size_t>(1);
+    std::vector<int2> tab(fill_at + 2, make_int2(0, INT32_MIN));
+    tab[fill_at] = tab[fill_at + 1] = make_int2(fill, fill);
+    for (int32_t i = 0; i < nc; ++i) {
+        const GcClassDesc &d = classes[i];
+        const int32_t K = d.kh * d.kw * cin;
+        gc->gather_bytes = std::max(gc->gather_bytes, static_cast<size_t>(p.cls[i].M) * static_cast<size_t>((K + 15) & ~15));
+        for (int32_t k = 0; k < K; k += p.gran) {
+            const int32_t tap = k / cin, c = k - tap * cin, ky = tap / d.kw, kx = tap - ky * d.kw;
+            const int32_t dy = ky * d.dy, dx = kx * d.dx;
+            const int64_t off = (static_cast<int64_t>(dy) * g.w + dx) * cin + c;
+            if (off > INT32_MAX || off < INT32_MIN) return ENN_B200_INVALID_PARAMS;
+            tab[static_cast<size_t>(p.cls[i].tab0 + k / p.gran)] = make_int2(static_cast<int>(off), (dy << 16) | (dx & 0xffff));
+        }
+        for (int32_t n = 0; n < N; ++n) {
+            int8_t *dst = wb.data() + ((static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + n % p.bn_data) * k_pad;
+            int64_t wsum = 0, wabs = 0;
+            for (int32_t k = 0; k < K; ++k) {
+                const uint8_t raw = weight(i, n, k);
+                const int32_t wv = g.w_signed ? static_cast<int32_t>(static_cast<int8_t>(raw)) : static_cast<int32_t>(raw) - 128;
+                dst[k] = static_cast<int8_t>(wv);
+                wsum += wv;
+                wabs += wv < 0 ? -wv : wv;
+            }
+            folds[static_cast<size_t>(i) * N + n] = fold_column(g, qh.bias[n], K, wsum, wabs, p.zw_eff);
+        }
+        if (p.need_asum)        // the all-ones row of every N tile: sum_k a
+            for (int32_t tn = 0; tn < tiles_n; ++tn) {
+                int8_t *dst = wb.data() + ((static_cast<size_t>(i) * tiles_n + tn) * p.bn_rows + p.bn_data) * k_pad;
+                for (int32_t k = 0; k < K; ++k) dst[k] = 1;
+            }
+    }
+    p.mode = column_mode(ctx, g, qh, folds, N, true);
+    p.sat_plain = column_sat_plain(ctx, g, p.mode);
+    std::vector<ColParam> cols(static_cast<size_t>(nc) * tiles_n * p.bn_rows, ColParam{});
+    for (int32_t i = 0; i < nc; ++i)
+        for (int32_t n = 0; n < N; ++n)
+            if (!column_constants(g, p.mode, qh.mult[n], qh.shift[n], folds[static_cast<size_t>(i) * N + n],
+                                  &cols[(static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + n % p.bn_data]))
+                p.mode = kModeGeneral;
+    cudaError_t e;
+    if ((e = cudaMalloc(&gc->w_dev, wb.size())) != cudaSuccess || (e = cudaMalloc(&gc->cols_dev, cols.size() * sizeof(ColParam))) != cudaSuccess ||
+        (e = cudaMalloc(&gc->tab_dev, tab.size() * sizeof(int2))) != cudaSuccess ||
+        (e = cudaMemcpy(gc->w_dev, wb.data(), wb.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(gc->cols_dev, cols.data(), cols.size() * sizeof(ColParam), cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemcpy(gc->tab_dev, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice)) != cudaSuccess || (e = gconv_init()) != cudaSuccess) {
+        ctx->last_error = std::string("gather convolution plan: ") + cudaGetErrorString(e);
+        return ENN_B200_CUDA_FAILURE;
+    }
+    p.cols = static_cast<const ColParam *>(gc->cols_dev);
+    p.tab = static_cast<const int2 *>(gc->tab_dev);
+    p.fill_src = reinterpret_cast<const uint8_t *>(p.tab + fill_at);
+    if (!encode_2d(ctx, &gc->map_b, gc->w_dev, static_cast<uint64_t>(k_pad), static_cast<uint64_t>(nc) * tiles_n * p.bn_rows, static_cast<uint64_t>(k_pad), kBK,
+                   static_cast<uint32_t>(p.bn_rows))) {
+        ctx->last_error = "cuTensorMapEncodeTiled failed for the weight tensor";
+        return ENN_B200_CUDA_FAILURE;
+    }
+    return ENN_B200_SUCCESS;
+}
+
 void free_plan(TcPlan *plan) {
     if (!plan) return;
     for (auto &gm : plan->gemms) {
         if (gm.w_dev) cudaFree(gm.w_dev);
         if (gm.cols_dev) cudaFree(gm.cols_dev);
         if (gm.ktab_dev) cudaFree(gm.ktab_dev);
+    }
+    if (plan->gc) {
+        if (plan->gc->w_dev) cudaFree(plan->gc->w_dev);
+        if (plan->gc->cols_dev) cudaFree(plan->gc->cols_dev);
+        if (plan->gc->tab_dev) cudaFree(plan->gc->tab_dev);
     }
     if (plan->scratch) cudaFree(plan->scratch);
     if (plan->err_host) cudaFreeHost(plan->err_host);
@@ -2076,6 +1821,30 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         return ENN_B200_SUCCESS;
     };
 
+    // Plans the operator as one gather convolution; on success the plan is complete.
+    auto try_gconv = [&](const std::vector<GcClassDesc> &classes, int32_t sy, int32_t sx, int64_t sn, int64_t s_y, int64_t s_x, auto wfn) -> int32_t {
+        std::unique_ptr<GcPlan> gc(new (std::nothrow) GcPlan());
+        if (!gc) return bail(ENN_B200_FAILURE);
+        plan->gc = std::move(gc);
+        const int32_t s2 = build_gconv(ctx, g, qh, classes, sy, sx, sn, s_y, s_x, wfn, plan->gc.get());
+        if (s2 == ENN_B200_INVALID_PARAMS) {
+            plan->gc.reset();       // nothing was allocated
+            return s2;
+        }
+        if (s2 != ENN_B200_SUCCESS) return bail(s2);
+        plan->gemms.clear();
+        if (cudaHostAlloc(reinterpret_cast<void **>(&plan->err_host), sizeof(int32_t), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(reinterpret_cast<void **>(&plan->err_dev), plan->err_host, 0) != cudaSuccess) {
+            ctx->last_error = "tensor-core plan: error word allocation failed";
+            return bail(ENN_B200_CUDA_FAILURE);
+        }
+        *plan->err_host = 0;
+        plan->gc->prm.err = plan->err_dev;
+        op->info.kernel_launches = 1;
+        op->tc = plan;
+        return ENN_B200_SUCCESS;
+    };
+
     if (op->kind != OP_DECONV) {
         const int64_t M64 = static_cast<int64_t>(g.n) * g.oh * g.ow;
         if (M64 <= 0 || M64 > INT32_MAX) return bail(ENN_B200_INVALID_PARAMS);
@@ -2162,6 +1931,12 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             ig.oh = g.oh; ig.ow = g.ow; ig.kh = g.kh; ig.kw = g.kw;
             ig.sy = g.sh; ig.sx = g.sw; ig.dy = g.dh; ig.dx = g.dw; ig.y0 = -g.pt; ig.x0 = -g.pl;
             ig.fill = fill;
+            if (!ctx->opt("no_gconv")) {
+                GcClassDesc cd{g.oh, g.ow, g.kh, g.kw, g.dh, g.dw, -g.pt, -g.pl, 0};
+                st = try_gconv({cd}, g.sh, g.sw, static_cast<int64_t>(g.oh) * g.ow * N, static_cast<int64_t>(g.ow) * N, N,
+                               [&](int32_t, int32_t n, int32_t k) { return weight(n, k); });
+                if (st != ENN_B200_INVALID_PARAMS) return st;
+            }
             st = make_conv_gemm(gm, ig, weight);
             if (st != ENN_B200_SUCCESS) return bail(st);
             if (gm.implicit) {
@@ -2180,6 +1955,34 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         // (oy + pad_t) % sh == py only ever meet kernel rows ky = py + sh * jy, so each class (py, px) is a
         // stride-1 correlation over the input with its own small filter:
         //   out[n, sh*q - pad_t + py, ...] = sum_{jy,jx,c} in[n, q - jy, r - jx, c] * w[c][co][py + sh*jy][px + sw*jx].
+        if (!ctx->opt("no_gconv")) {
+            struct Cls { int32_t py, px, jx_e; bool empty; };
+            std::vector<GcClassDesc> cds;
+            std::vector<Cls> info;
+            for (int32_t py = 0; py < g.sh; ++py)
+                for (int32_t px = 0; px < g.sw; ++px) {
+                    const int32_t jy_n = py < g.kh ? (g.kh - py + g.sh - 1) / g.sh : 0, jx_n = px < g.kw ? (g.kw - px + g.sw - 1) / g.sw : 0;
+                    const int32_t q_lo = (g.pt - py + g.sh - 1 >= 0) ? (g.pt - py + g.sh - 1) / g.sh : 0;
+                    const int32_t q_hi = (g.oh - 1 + g.pt - py) >= 0 ? (g.oh - 1 + g.pt - py) / g.sh : -1;
+                    const int32_t r_lo = (g.pl - px + g.sw - 1 >= 0) ? (g.pl - px + g.sw - 1) / g.sw : 0;
+                    const int32_t r_hi = (g.ow - 1 + g.pl - px) >= 0 ? (g.ow - 1 + g.pl - px) / g.sw : -1;
+                    if (q_hi < q_lo || r_hi < r_lo) continue;
+                    const bool empty = jy_n == 0 || jx_n == 0;      // outputs without taps: one zero-weight dummy tap
+                    const int32_t oy0 = g.sh * q_lo - g.pt + py, ox0 = g.sw * r_lo - g.pl + px;
+                    cds.push_back({q_hi - q_lo + 1, r_hi - r_lo + 1, jy_n > 0 ? jy_n : 1, jx_n > 0 ? jx_n : 1, -1, -1, q_lo, r_lo,
+                                   (static_cast<int64_t>(oy0) * g.ow + ox0) * N});
+                    info.push_back({py, px, jx_n > 0 ? jx_n : 1, empty});
+                }
+            st = try_gconv(cds, 1, 1, static_cast<int64_t>(g.oh) * g.ow * N, static_cast<int64_t>(g.sh) * g.ow * N, static_cast<int64_t>(g.sw) * N,
+                           [&](int32_t i, int32_t n, int32_t k) -> uint8_t {
+                               const Cls &ci = info[static_cast<size_t>(i)];
+                               if (ci.empty) return static_cast<uint8_t>(g.w_zp);
+                               const int32_t tap = k / cin, c = k - tap * cin, jy = tap / ci.jx_e, jx = tap - jy * ci.jx_e;
+                               const int32_t ky = ci.py + g.sh * jy, kx = ci.px + g.sw * jx;
+                               return w[((static_cast<size_t>(ky) * g.kw + kx) * cin + c) * N + n];
+                           });
+            if (st != ENN_B200_INVALID_PARAMS) return st;
+        }
         plan->gemms.reserve(static_cast<size_t>(g.sh) * g.sw);
         for (int32_t py = 0; py < g.sh; ++py) {
             for (int32_t px = 0; px < g.sw; ++px) {
@@ -2336,6 +2139,18 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
 // INVALID_PARAMS when this plan cannot take it; the caller then keeps the two operators.
 int32_t tc_fuse_add(enn_b200_op *op, const AddParams &add, bool conv_is_second) {
     TcPlan *plan = static_cast<TcPlan *>(op->tc);
+    if (plan && plan->gc && !plan->fused_add) {
+        GcParams &p = plan->gc->prm;
+        if (op->kind != OP_CONV || (p.mode != kModeNudge && p.mode != kModeGeneral) || (p.N & 15) != 0 || !add.lut || add.is_signed != p.a_signed)
+            return ENN_B200_INVALID_PARAMS;
+        if (plan->gc->smem_bytes + 2048 > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
+        plan->gc->smem_bytes += 2048;
+        p.add = add;
+        p.add_on = 1;
+        p.add_swap = conv_is_second ? 1 : 0;
+        plan->fused_add = true;
+        return ENN_B200_SUCCESS;
+    }
     if (!plan || plan->gemms.size() != 1 || plan->fused_add) return ENN_B200_INVALID_PARAMS;
     TcGemm &gm = plan->gemms[0];
     TcParams &p = gm.prm;
@@ -2357,6 +2172,40 @@ void tc_set_residual(enn_b200_op *op, const void *res) {
     if (TcPlan *plan = static_cast<TcPlan *>(op->tc)) plan->residual = static_cast<const uint8_t *>(res);
 }
 
+namespace {
+int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) {
+    enn_b200_context *ctx = op->ctx;
+    GcParams &p = plan->gc->prm;
+    if ((reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(p.gran - 1)) != 0) {
+        // sub-buffers at odd offsets: the general kernels take any alignment
+        if (plan->fused_add) {
+            ctx->last_error = "fused convolution + add needs 16-byte aligned pointers";
+            return ENN_B200_INVALID_PARAMS;
+        }
+        const cudaError_t e = op->kind == OP_DECONV ? launch_deconv_direct(op->g, op->rq, in, op->w_direct, out, ctx->stream)
+                                                    : launch_conv_direct(op->g, op->rq, in, op->w_direct, out, ctx->stream);
+        if (e == cudaSuccess) return ENN_B200_SUCCESS;
+        ctx->last_error = std::string("kernel launch: ") + cudaGetErrorString(e);
+        return ENN_B200_CUDA_FAILURE;
+    }
+    if (plan->fused_add) {
+        if (!plan->residual || ((reinterpret_cast<uintptr_t>(plan->residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) {
+            ctx->last_error = "fused convolution + add needs the second addend and 16-byte aligned pointers";
+            return ENN_B200_INVALID_PARAMS;
+        }
+        p.add_res = plan->residual;
+    }
+    p.in = static_cast<const uint8_t *>(in);
+    p.out = static_cast<uint8_t *>(out);
+    p.test_starve = plan->starve_next ? 1 : 0;
+    plan->starve_next = false;
+    const cudaError_t e = gconv_launch(*plan->gc, ctx->stream);
+    if (e == cudaSuccess) return ENN_B200_SUCCESS;
+    ctx->last_error = std::string("gconv_kernel launch: ") + cudaGetErrorString(e);
+    return ENN_B200_CUDA_FAILURE;
+}
+}  // namespace
+
 int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
     TcPlan *plan = static_cast<TcPlan *>(op->tc);
     enn_b200_context *ctx = op->ctx;
@@ -2367,6 +2216,7 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = buf;
         return ENN_B200_CUDA_FAILURE;
     }
+    if (plan->gc) return gconv_execute(op, plan, in, out);
     #ifdef ENN_B200_DEV
     const bool fan_out = plan->fan_out && !getenv("ENN_B200_TC_DEBUG");
 #else
@@ -2551,7 +2401,7 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = "enn_b200_op_execute_noalloc: the operator is not bound to the tensor-core path (or has a fused add)";
         return ENN_B200_INVALID_PARAMS;
     }
-    size_t need = 0;
+    size_t need = plan->gc ? plan->gc->gather_bytes : 0;
     for (auto &gm : plan->gemms) {
         if (!gm.gather) {
             ctx->last_error = "enn_b200_op_execute_noalloc: this operator has no gathered input matrix; call enn_b200_op_execute";
@@ -2566,6 +2416,11 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
                       need, kStaticScratchBytes);
         ctx->last_error = buf;
         return ENN_B200_INVALID_PARAMS;
+    }
+    if (plan->gc) {      // gathers into shared memory: no scratch array needed
+        if (*plan->err_host == 0) return gconv_execute(op, plan, in, out);
+        ctx->last_error = "gather convolution gave up on a barrier wait earlier";
+        return ENN_B200_CUDA_FAILURE;
     }
     if (ctx->device < 0 || ctx->device >= 64) return ENN_B200_INVALID_PARAMS;
     uint8_t *scratch = nullptr;

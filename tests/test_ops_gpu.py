@@ -1191,3 +1191,49 @@ def test_oplist_with_graph_operators(enn, orc, ctx):
             assert np.array_equal(y, y6.reshape(-1))
     finally:
         ol.destroy()
+
+
+# Gather convolution: 16-, 8- and 4-byte copies; weights resident and travelling with the stages; one and two accumulator
+# buffers; several N tiles (with more columns than are staged at once); ragged M, N and K tails; several units per CTA.
+GCONV_CASES = {
+    "g16_resident_tail_k": ("conv", dict(n=3, h=17, w=15, cin=48, cout=20, k=3, stride=2, w_zp=131, out_scale=0.05)),
+    "g16_staged_wide": ("conv", dict(n=2, h=9, w=11, cin=176, cout=240, k=3, per_channel=True, out_scale=0.6)),
+    "g16_many_columns": ("conv", dict(n=1, h=6, w=5, cin=32, cout=1100, k=3, per_channel=True, out_scale=0.4, act=cases.enn.ACT_NONE)),
+    "g16_many_units": ("conv", dict(n=9, h=97, w=65, cin=16, cout=16, k=3, per_channel=True, out_scale=0.0235, out_zp=0)),
+    "g8_k_tail": ("conv", dict(n=2, h=21, w=19, cin=24, cout=36, k=3, dil=2, w_zp=119, out_scale=0.05)),
+    "g8_pointwise_s8": ("conv", dict(n=2, h=13, w=13, cin=72, cout=200, k=1, per_channel=True, act_dtype=cases.enn.S8, in_zp=-7, out_zp=4, out_scale=0.5)),
+    "g4_5x5_odd_n": ("conv", dict(n=1, h=12, w=14, cin=20, cout=33, k=5, per_channel=True, out_scale=0.4)),
+    "deconv_g8_four_classes": ("deconv", dict(n=2, h=11, w=9, cin=40, cout=24, per_channel=True, out_scale=0.5)),
+    "deconv_g4_stride3": ("deconv", dict(n=1, h=7, w=6, cin=12, cout=17, k=4, stride=3, pad=1)),
+    "deconv_g16_staged": ("deconv", dict(n=5, h=20, w=23, cin=160, cout=136)),
+    "deconv_taps_missing": ("deconv", dict(n=1, h=5, w=5, cin=16, cout=8, k=2, stride=3, pad=0)),
+}
+
+
+@pytest.mark.parametrize("name", list(GCONV_CASES))
+def test_gather_convolution(enn, orc, ctx, name):
+    kind, kw = GCONV_CASES[name]
+    mk, ref, case = (enn.conv2d, orc.conv2d, cases.conv_case) if kind == "conv" else (enn.deconv, orc.deconv, cases.deconv_case)
+    d, x, w, b, sc = case(seed=_seed("gconv_" + name), **kw)
+    y_ref = ref(d, x, w, b, sc)
+    op = mk(ctx, d, w, b, sc)
+    try:
+        assert op.info.impl == enn.IMPL_TCGEN05 and op.info.kernel_launches == 1
+        _check(op, y_ref, x)
+        buf = ctx.malloc(x.nbytes + 32)              # a sub-buffer at an odd offset: the general kernel takes it
+        out = ctx.malloc(y_ref.size)
+        pin = type(buf)(buf.value + 1)
+        ctx.upload(pin, x)
+        op.execute(pin, out)
+        assert np.array_equal(ctx.download(out, (y_ref.size,), y_ref.dtype), y_ref.reshape(-1))
+        ctx.free(buf)
+        ctx.free(out)
+        op.test_starve_next()                        # the bounded waits of all roles end, and the operator works afterwards
+        op.run(x)
+        ctx.sync()
+        with pytest.raises(enn.EnnError):
+            op.run(x)
+        op.clear_error()
+        _check(op, y_ref, x)
+    finally:
+        op.release()
