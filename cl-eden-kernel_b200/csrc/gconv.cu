@@ -313,15 +313,10 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
         }
     } else {
         // ---------------- epilogue ----------------
-        const int row_in_tile = warp * 32 + lane;
-        const int32_t hi_clamp = p.act_max - p.act_min;
-        const uint32_t sign_word = p.a_signed ? 0x80808080u : 0u;
-        const uint32_t lo_word = (static_cast<uint32_t>(p.act_min + (p.a_signed ? 128 : 0)) & 0xff) * 0x01010101u;
-        constexpr bool kPlainPack = MODE == kModeReluSat;
         int64_t st_bits = p.out_sn | p.out_sy | p.out_sx | p.bn_data | static_cast<int64_t>(reinterpret_cast<uintptr_t>(p.out));
         for (int c = 0; c < p.n_classes; ++c) st_bits |= p.cls[c].out_base;
-        const int st_align = (st_bits & 15) == 0 ? 16 : ((st_bits & 7) == 0 ? 8 : ((st_bits & 3) == 0 ? 4 : 1));
-        const int cps = p.bn_data >> 4;
+        const EpiArgs e = epi_args(p, st_bits, FADD ? p.add_res - p.out : 0, fadd);
+        EpiTile t;
         int loaded = -1;
         uint32_t it = 0;
         bool ok = true;
@@ -342,77 +337,32 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
                 asm volatile("bar.sync 2, %0;" ::"n"(32 * kEpiWarpsGc) : "memory");
                 loaded = ct;
             }
-            const uint8_t *cols = sp + L.cols + (p.cols_all ? static_cast<size_t>(ct) * p.bn_rows * 16 : 0);
-            const uint32_t m = static_cast<uint32_t>(u.tm * kBM + row_in_tile);
-            const bool row_ok = m < static_cast<uint32_t>(c.M);
-            const int n_base = u.tn * p.bn_data, n_cols = min(p.bn_data, p.N - n_base);
-            uint8_t *orow = p.out + c.out_base + n_base;
-            if (row_ok) {
-                const uint32_t img = c.div_img.div(m), rem = m - img * static_cast<uint32_t>(c.oh * c.ow);
-                const uint32_t oy = c.div_ow.div(rem), ox = rem - oy * static_cast<uint32_t>(c.ow);
-                orow += img * p.out_sn + oy * p.out_sy + ox * p.out_sx;
+            const uint8_t *cols = sp + L.cols + (p.cols_all ? ct * p.bn_rows * 16 : 0);
+            // Lane l works out where row l of the warp's quarter starts; a thread then takes its four rows from the lanes.
+            const int n_base = u.tn * p.bn_data;
+            t.n_left = min(p.bn_data, p.N - n_base);
+            {
+                const uint32_t m = static_cast<uint32_t>(u.tm * kBM + warp * 32 + lane);
+                int64_t off = -1;
+                if (m < static_cast<uint32_t>(c.M)) {
+                    const uint32_t img = c.div_img.div(m), rem = m - img * static_cast<uint32_t>(c.oh * c.ow);
+                    const uint32_t oy = c.div_ow.div(rem), ox = rem - oy * static_cast<uint32_t>(c.ow);
+                    off = c.out_base + n_base + img * p.out_sn + oy * p.out_sy + ox * p.out_sx;
+                }
+                t.live = 0;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const int64_t o = __shfl_sync(0xffffffffu, off, (lane >> 2) + 8 * h);
+                    t.live |= o >= 0 ? 1u << h : 0u;
+                    t.row[h] = p.out + o;
+                }
             }
-            const ptrdiff_t res_delta = FADD ? p.add_res - p.out : 0;
             if (ok) ok = mbar_wait(tfull0 + 8 * ab, use & 1, abort_flag, p.err, 4);
             if (!ok) continue;
             tc_fence_after();
             const uint32_t t_row = tmem_base + ab * p.bn_rows + (static_cast<uint32_t>(warp * 32) << 16);
-            int32_t asum_term = 0;
-            if (ASUM) {
-                uint32_t rs;
-                tmem_ld_x1(t_row + p.bn_data, rs);
-                tmem_ld_wait();
-                asum_term = p.zw_eff * static_cast<int32_t>(rs);
-            }
-            auto chunk = [&](const uint32_t (&r)[16], int c0) {
-                uint32_t w[4];
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    int32_t y[4];
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        ColRegs cv;
-                        ld_col_shared<MODE>(cols + (c0 + jj * 4 + b) * 16, cv);
-                        int32_t acc = static_cast<int32_t>(r[jj * 4 + b]);
-                        if (ASUM) acc -= asum_term;
-                        y[b] = tc_requant<MODE>(acc, cv, hi_clamp, p.out_zp, p.act_min, p.act_max);
-                    }
-                    const uint32_t hi = pack_sat_u8_tc(y[3], y[2], 0);
-                    const uint32_t pk = pack_sat_u8_tc(y[1], y[0], hi);
-                    w[jj] = kPlainPack ? pk : ((pk + lo_word) ^ sign_word);
-                }
-                if (!row_ok) return;
-                if constexpr (FADD) fadd_chunk(w, orow + c0 + res_delta, fadd);
-                const int left = n_cols - c0;
-                if (st_align == 16 && left >= 16) {
-                    *reinterpret_cast<uint4 *>(orow + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                } else if (st_align >= 8 && (left & 7) == 0) {
-                    *reinterpret_cast<uint2 *>(orow + c0) = make_uint2(w[0], w[1]);
-                    if (left >= 16) *reinterpret_cast<uint2 *>(orow + c0 + 8) = make_uint2(w[2], w[3]);
-                } else if (st_align >= 4 && (left & 3) == 0) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (4 * q < left) *reinterpret_cast<uint32_t *>(orow + c0 + 4 * q) = w[q];
-                } else {
-#pragma unroll
-                    for (int b = 0; b < 16; ++b)
-                        if (b < left) orow[c0 + b] = static_cast<uint8_t>(w[b >> 2] >> (8 * (b & 3)));
-                }
-            };
-            // Accumulator loads one chunk ahead of the arithmetic.
-            uint32_t ra[16], rb[16];
-            const int n_chunks = min(cps, (n_cols + 15) >> 4);
-            tmem_ld_x16(t_row, ra);
-            for (int ch = 0; ch < n_chunks; ch += 2) {
-                tmem_ld_wait();
-                if (ch + 1 < n_chunks) tmem_ld_x16(t_row + 16 * (ch + 1), rb);
-                chunk(ra, 16 * ch);
-                if (ch + 1 < n_chunks) {
-                    tmem_ld_wait();
-                    if (ch + 2 < n_chunks) tmem_ld_x16(t_row + 16 * (ch + 2), ra);
-                    chunk(rb, 16 * (ch + 1));
-                }
-            }
+            if (ASUM) epi_asum(t_row, p.bn_data, p.zw_eff, lane, t.asum);
+            epi_tile<MODE, ASUM, FADD>(t_row, 0, 1, p.bn_data, t, lane, e, [&](int) { return cols; });
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty0 + 8 * ab);

@@ -61,7 +61,8 @@ namespace {
 // chunk) run the MobileNetV2 graph 6 % faster than 24 warps capped at 72 registers; 8 and 16 warps are 1 % behind.
 constexpr int kEpiWarps = 8;
 constexpr int kColGroups = kEpiWarps / 4;
-constexpr int kChunksPerWarp = (kMaxBN / 16 + kColGroups - 1) / kColGroups;   // chunks one warp can own
+constexpr int kGroupsPerWarp = kMaxBN / 32 / kColGroups;   // column groups one warp can own
+constexpr int kColEntries = kEpiWarps * kGroupsPerWarp * 32;   // column constants staged in shared memory
 // Warp 0 loads the A tiles, warp 1 issues the MMAs, warps 2 .. kEpiWarps + 1 are the epilogue (warp & 3 is the TMEM lane
 // quarter a warp may read); long-K GEMMs are launched with one more warp that loads the B tiles.
 // 128 registers per thread is the ceiling for this shape: a scheduler with four resident warps has 16384 registers.
@@ -81,7 +82,7 @@ struct TcParams {
     int32_t bn_data;        // real output columns per N tile
     int32_t stages;
     int32_t kpack;          // k-blocks that share one pipeline stage (one barrier round trip per kpack k-blocks)
-    int32_t b_res;          // implicit convolutions: the whole B operand (one N tile, every tap) is loaded once and stays in shared memory
+    int32_t b_res;          // the whole B operand (one N tile) is loaded once and stays in shared memory
     int32_t need_asum;      // 1: column bn_data of each accumulator tile holds sum_k a
     int32_t zw_eff;         // zw'
     int32_t a_signed;
@@ -95,19 +96,12 @@ struct TcParams {
     // out + out_base + img * out_sn + qy * out_sy + qx * out_sx.  A plain [M][N] result uses qh = 1, qw = M.
     int32_t qh, qw;
     int64_t out_base, out_sn, out_sy, out_sx;
-    // Implicit-convolution mode (taps > 0): an M tile is a patch of conv_ht x conv_wt output positions of one image;
-    // k-block kb = (tap, channel chunk) and its A tile is the 4-D box {span channels, conv_wt, conv_ht, 1} of the
-    // (zero-point padded) NHWC input at (chunk * span, tx * conv_wt + tap_dx, ty * conv_ht + tap_dy, image).
-    int32_t taps, cchunks;
-    int32_t conv_ht, conv_wt, conv_ty, conv_tx;
     int32_t span;           // bytes of K per k-block = swizzle span of both operand tiles: 128, 64 or 32
     int32_t k_pad;          // row pitch of the packed B matrix (K rounded up to 128)
-    int16_t tap_dx[64], tap_dy[64];
     int32_t *err;           // host-mapped error word
     long long *dbg;         // optional per-CTA cycle counters [grid][8] (null in normal use)
     int32_t dbg_mode;       // development switches (0 in normal use)
     int32_t sat_plain;      // kModeReluHi whose clamp is [0, 255] on unsigned bytes: run the kModeReluSat kernel
-    int32_t no_wide_store;  // tuning: keep 16-byte stores
     // Fused quantized add (kernels with FADD): the add operator's parameters and stage-1 tables (2 x 256 words, staged in
     // shared memory at add_off), the other addend (same layout as the output), and which addend the convolution's result is.
     AddParams add;
@@ -115,7 +109,6 @@ struct TcParams {
     const uint8_t *add_res;
     int32_t add_off;
     int32_t add_swap;       // 1: the convolution result is the add's second input
-    int32_t epi_g;          // M tiles of a work unit the epilogue requantises together per column (1, 2 or 4)
     int32_t test_starve;    // self-test of the bounded waits: no operand copy is issued and the waits give up early
 };
 
@@ -211,7 +204,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t s_cols_u32 = smem_u32(s_cols);
     // The same place as a pointer that is visibly derived from the shared array (for loads written in C++).
     const uint8_t *s_cols_sp = smem_raw + (s_cols_u32 - smem_u32(smem_raw));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(s_cols + kEpiWarps * kChunksPerWarp * 16);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(s_cols + kColEntries);
     // bars: full[stages], empty[stages], tmem_full[2], tmem_empty[2]
     const int nst = p.stages;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * nst + 5);      // bars[2 * nst + 4]: resident B loaded
@@ -243,7 +236,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // Column constants: when those of all N tiles fit the staging area they are loaded here once, shared by every
     // epilogue warp (any warp can then take any chunk); otherwise each epilogue warp keeps private copies of the
     // columns it owns and refreshes them when the N tile changes.
-    const bool cols_shared = p.tiles_n * p.bn_rows <= kEpiWarps * kChunksPerWarp * 16;
+    const bool cols_shared = p.tiles_n * p.bn_rows <= kColEntries;
     if (cols_shared)
         for (int i = threadIdx.x; i < p.tiles_n * p.bn_rows; i += blockDim.x) s_cols[i] = __ldg(reinterpret_cast<const int4 *>(p.cols) + i);
     FaddCtx fadd{};
@@ -283,7 +276,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // thread issues about one tensor copy per 420 cycles, which is also about what the tensor pipe needs per
         // k-block, so two lanes of each producer warp take the k-blocks in turn (two lanes issuing in step reach
         // 1.7 x the rate of one).  A stage always belongs to the same lane, so each lane meets its stages' phases in order.
-        const bool pair_lanes = !starve && split && p.taps == 0 && p.group == 1 && p.kpack == 1 && (nst & 1) == 0 && p.k_blocks >= 8 &&
+        const bool pair_lanes = !starve && split && p.group == 1 && p.kpack == 1 && (nst & 1) == 0 && p.k_blocks >= 8 &&
                                 !(ENN_DBG_MODE(p) & 9);
         if (pair_lanes) {
             const int nl = 2;      // lanes that share the issue (four measured slightly worse than two)
@@ -326,13 +319,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             }
         } else if (!starve && !TWO && !split && bres && (nst & 1) == 0 && !(ENN_DBG_MODE(p) & 9)) {
-            // Resident weights (implicit convolutions, narrow pointwise layers): only A tiles are left to load, and the copy
+            // Resident weights (narrow pointwise layers): only A tiles are left to load, and the copy
             // issue rate of one thread still bounds the kernel, so lanes 0 and 1 fill alternate stages (a stage keeps its lane).
             if (lane < 2) {
-                const uint32_t a_tx = p.taps > 0 ? static_cast<uint32_t>(p.conv_ht * p.conv_wt) * span : a_bytes;
                 const uint32_t sa0 = smem_u32(tiles);
                 const int gpt = (p.k_blocks + p.kpack - 1) / p.kpack;      // stages per M tile
-                const int per_img = p.taps > 0 ? p.conv_ty * p.conv_tx : 1;
                 int tile = tile_first, j = 0, g = 0, tg = 0, tn = 0, nsub = 0;
                 bool done = tile >= total_tiles, ok = true;
                 if (!done) {
@@ -356,31 +347,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 };
                 advance(lane);
                 uint32_t stage = static_cast<uint32_t>(lane), phase = 0;
-                int tm_cur = -1, img = 0, ty = 0, tx = 0;
                 while (!done) {
                     const int tm = tg * p.group + j;
-                    if (tm != tm_cur && p.taps > 0) {          // patch (img, ty, tx) of the output grid
-                        img = tm / per_img;
-                        const int rem = tm - img * per_img;
-                        ty = rem / p.conv_tx;
-                        tx = rem - ty * p.conv_tx;
-                    }
-                    tm_cur = tm;
                     const int kb0 = g * p.kpack, nkb = min(p.kpack, p.k_blocks - kb0);
                     const uint32_t ebar = empty0 + 8 * stage;
                     if (!mbar_test_wait(ebar, phase ^ 1) && !mbar_wait_fast(ebar, phase ^ 1, abort_flag, p.err, 1)) { ok = false; break; }
                     const uint32_t bar = full0 + 8 * stage;
-                    mbar_expect_tx(bar, a_tx * nkb);
+                    mbar_expect_tx(bar, a_bytes * nkb);
                     uint32_t sa = sa0 + stage * stage_bytes;
-                    if (p.taps > 0) {
-                        int tap = kb0 / p.cchunks, cc = kb0 - tap * p.cchunks;
-                        for (int q = 0; q < nkb; ++q, sa += kb_bytes) {
-                            tma_load_4d(sa, &map_a, bar, cc * static_cast<int>(span), tx * p.conv_wt + p.tap_dx[tap], ty * p.conv_ht + p.tap_dy[tap], img);
-                            if (++cc == p.cchunks) { cc = 0; ++tap; }
-                        }
-                    } else {
-                        for (int q = 0; q < nkb; ++q, sa += kb_bytes) tma_load_2d(sa, &map_a, bar, (kb0 + q) * static_cast<int>(span), tm * kBM);
-                    }
+                    for (int q = 0; q < nkb; ++q, sa += kb_bytes) tma_load_2d(sa, &map_a, bar, (kb0 + q) * static_cast<int>(span), tm * kBM);
                     stage += 2;
                     if (stage >= static_cast<uint32_t>(nst)) { stage -= nst; phase ^= 1; }
                     advance(2);
@@ -400,8 +375,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const uint32_t sa_stage0 = smem_u32(tiles);
                 uint32_t sa_stage = sa_stage0;
                 // bytes this producer's loads add to a k-block (pairs: of both CTAs, counted on rank 0's barrier)
-                const uint32_t a_tx = p.taps > 0 ? static_cast<uint32_t>(p.conv_ht * p.conv_wt) * span : a_bytes;
-                const uint32_t kb_tx = ((DO_A ? a_tx : 0u) + (DO_B && !bres ? b_bytes : 0u)) * (TWO ? 2u : 1u);
+                const uint32_t kb_tx = ((DO_A ? a_bytes : 0u) + (DO_B && !bres ? b_bytes : 0u)) * (TWO ? 2u : 1u);
                 bool ok = true;
                 long long t_wait = 0;
                 for (int tile = tile_first; tile < total_tiles && ok; tile += tile_step) {
@@ -410,15 +384,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const int nsub = min(p.group, p.tiles_m - tg * p.group);
                     for (int j = 0; j < nsub && ok; ++j) {
                         const int tm = TWO ? tg * 2 + static_cast<int>(rank) : tg * p.group + j;
-                        int img = 0, ty = 0, tx = 0;
-                        if (DO_A && p.taps > 0) {       // patch (img, ty, tx) of the output grid
-                            const int per_img = p.conv_ty * p.conv_tx;
-                            img = tm / per_img;
-                            const int rem = tm - img * per_img;
-                            ty = rem / p.conv_tx;
-                            tx = rem - ty * p.conv_tx;
-                        }
-                        int tap = 0, cc = 0;
                         const int row_a = tm * kBM;
                         const int row_b = tn * p.bn_rows + (TWO ? static_cast<int>(rank) * (p.bn_rows >> 1) : 0);
                         const int kstep_b = static_cast<int>(span);
@@ -444,14 +409,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             } else {
                                 mbar_expect_tx(bar, kb_tx * nkb);
                                 for (int q = 0; q < nkb; ++q, sa += kb_bytes) {
-                                    if (DO_A) {
-                                        if (p.taps > 0) {
-                                            tma_load_4d(sa, &map_a, bar, cc * static_cast<int>(span), tx * p.conv_wt + p.tap_dx[tap], ty * p.conv_ht + p.tap_dy[tap], img);
-                                            if (++cc == p.cchunks) { cc = 0; ++tap; }
-                                        } else {
-                                            tma_load_2d(sa, &map_a, bar, (kb0 + q) * kstep_b, row_a);
-                                        }
-                                    }
+                                    if (DO_A) tma_load_2d(sa, &map_a, bar, (kb0 + q) * kstep_b, row_a);
                                     if (DO_B && !bres) tma_load_2d(sa + a_bytes, &map_b, bar, (kb0 + q) * kstep_b, row_b);
                                 }
                             }
@@ -490,11 +448,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // K slices per k-block: the whole span, except that the last k-block of a plain GEMM stops after the slices
             // that hold real K (rounded up to 1, 2 or 4: the operands are zero beyond K, so a surplus slice adds nothing).
             const int ks = static_cast<int>(span >> 5);
-            int ks_last = ks;
-            if (p.taps == 0) {
-                const int real = (p.K - (p.k_blocks - 1) * static_cast<int>(span) + 31) >> 5;
-                ks_last = real <= 1 ? 1 : (real == 2 ? 2 : 4);
-            }
+            const int real = (p.K - (p.k_blocks - 1) * static_cast<int>(span) + 31) >> 5;
+            const int ks_last = real <= 1 ? 1 : (real == 2 ? 2 : 4);
             uint32_t lo_stage = lo0;
             const uint32_t bres_lo = smem_u32(b_resident) >> 4, bstride16 = b_stride >> 4;
             const uint32_t looks = starve ? 64u : (kSpinLimit >> 7);
@@ -563,32 +518,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else {
-        // ---------------- epilogue: thread = accumulator row, warp = (lane quarter, column share) ----------------
+        // ---------------- epilogue (tc_common.cuh): warp = (lane quarter, share of the column groups) ----------------
         const int q = warp & 3;                            // TMEM lane group this warp may access
-        const int cgrp = (warp - 2) >> 2;                  // which share of the 16-column chunks this warp takes
-        const int row_in_tile = q * 32 + lane;
-        const int32_t hi_clamp = p.act_max - p.act_min;
-        // The lower clamp is added back to the packed bytes.  Unsigned outputs: byte + act_min <= act_max <= 255, so a
-        // plain 32-bit add never carries between bytes.  Signed outputs (act_min may be negative): the bytes get
-        // act_min + 128 (0..127, sums again <= 255) and the sign bit of every byte is flipped afterwards.
-        const uint32_t sign_word = p.a_signed ? 0x80808080u : 0u;
-        const uint32_t lo_word = (static_cast<uint32_t>(p.act_min + (p.a_signed ? 128 : 0)) & 0xff) * 0x01010101u;
+        const int cgrp = (warp - 2) >> 2;                  // which share of the column groups this warp takes
         const int64_t st_bits = p.out_base | p.out_sn | p.out_sy | p.out_sx | p.bn_data | static_cast<int64_t>(reinterpret_cast<uintptr_t>(p.out));
-        const int st_align = (st_bits & 15) == 0 ? 16 : ((st_bits & 7) == 0 ? 8 : 1);   // widest store every row start allows
-        const bool st_fast = st_align == 16 && (p.N & 15) == 0;      // every chunk is one aligned 16-byte store
-        const bool whole_rows = st_fast && p.taps == 0 && !(ENN_DBG_MODE(p) & 4);   // rows of a full M tile are all real: see the chunk loop
-        const int patch_y = p.taps > 0 ? row_in_tile / p.conv_wt : 0;   // this thread's position in the output patch
-        const int patch_x = p.taps > 0 ? row_in_tile - patch_y * p.conv_wt : 0;
-        const int cps_mod = (p.bn_data >> 4) % kColGroups;
-        // Several M tiles of a unit requantised together (shared column constants): flat row-major outputs with aligned rows only.
-        const ptrdiff_t res_delta = FADD ? p.add_res - p.out : 0;      // other addend of a fused add: same offsets as the output
-        const bool flat = !TWO && st_fast && p.taps == 0 && p.qh == 1 && ENN_DBG_MODE(p) == 0;
-        // 32-byte stores: rows and pairs of chunks start on 32-byte boundaries, the constants of all columns are shared
-        const bool wide_ok = flat && (st_bits & 31) == 0 && (p.bn_data & 31) == 0 && cols_shared && !p.no_wide_store;
-        uint32_t wrot = 0;
-        const int epi_g = flat && p.epi_g > 1 ? p.epi_g : 0;      // 0: the one-tile loop below
-        const uint32_t rot_step = static_cast<uint32_t>((((p.group + max(epi_g, 1) - 1) / max(epi_g, 1)) * (p.bn_data >> 4)) % kColGroups);
+        const EpiArgs e = epi_args(p, st_bits, FADD ? p.add_res - p.out : 0, fadd);      // other addend of a fused add: same offsets as the output
+        EpiTile t;
+        const int ng = (p.bn_data + 31) >> 5;            // groups of 32 columns (the last one may have 16)
         uint32_t it = 0;
+        int turn = 0;                                    // column groups seen so far: they alternate between the shares
         bool ok = true;
         int loaded_tn = -1;
         long long t_tfull = 0, t_begin = dbg ? clock64() : 0;
@@ -598,19 +536,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int nsub = min(p.group, p.tiles_m - tg * p.group);
             const uint32_t ab = it & 1, use = it >> 1;
             const long long t0 = dbg ? clock64() : 0;
-            // Chunk c of the buffer = 16 columns cc of M tile j: c = j * cps + cc.  This warp owns chunks
-            // cgrp, cgrp + kColGroups, ...; it keeps private copies of the constants of the columns it meets.
-            const int cps = p.bn_data >> 4;
-            const uint32_t my_cols = s_cols_u32 + (warp - 2) * (kChunksPerWarp * 16 * 16);
+            // Constants of the N tile: staged for all warps when those of every tile fit, else each warp keeps private copies of
+            // the groups it owns (cgrp, cgrp + kColGroups, ...).
+            const uint32_t priv = static_cast<uint32_t>(warp - 2) * (kGroupsPerWarp * 512);
             if (!cols_shared && tn != loaded_tn) {
                 const int4 *src = reinterpret_cast<const int4 *>(p.cols + static_cast<size_t>(tn) * p.bn_rows);
                 __syncwarp();
-                for (int i = lane; i < kChunksPerWarp * 16; i += 32) {
-                    const int c = (i >> 4) * kColGroups + cgrp;
-                    if (c < p.group * cps) {
-                        const int4 v = __ldg(src + (c % cps) * 16 + (i & 15));
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(my_cols + i * 16), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-                    }
+                for (int g = cgrp, k = 0; g < ng; g += kColGroups, ++k) {
+                    const int c = g * 32 + lane;
+                    if (c < p.bn_data) s_cols[(priv >> 4) + k * 32 + lane] = __ldg(src + c);
                 }
                 __syncwarp();
                 loaded_tn = tn;
@@ -618,244 +552,44 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (!mbar_wait(tfull0 + 8 * ab, use & 1, abort_flag, p.err, 4)) { ok = false; break; }
             if (dbg) t_tfull += clock64() - t0;
             tc_fence_after();
-            const uint32_t t_row = tmem_base + ab * kMaxBN + (static_cast<uint32_t>(q * 32) << 16);
+            const uint32_t t_buf = tmem_base + ab * kMaxBN + (static_cast<uint32_t>(q * 32) << 16);
             const int n_base = tn * p.bn_data;
-            const int n_cols = min(p.bn_data, p.N - n_base);
-
-            // Walk this warp's chunks M tile by M tile: chunk c = j * cps + cc belongs to this warp when c = cgrp (mod
-            // kColGroups); `first` is the first such cc of M tile j and moves by -cps (mod kColGroups) from one M tile to
-            // the next.  Everything that depends only on the M tile (row pointer, row sum) is computed once per j.
-            // With shared constants the column groups that get one chunk more than the others change from tile to tile
-            // (the chunks of a buffer rarely divide evenly over the groups).
-            int first = cgrp;
-            if (cols_shared) {
-                first += static_cast<int>((it * rot_step) % kColGroups);
-                if (first >= kColGroups) first -= kColGroups;
-            }
-            uint32_t lc_private = my_cols;
-            const uint32_t lc_shared = s_cols_u32 + static_cast<uint32_t>(tn * p.bn_rows) * 16;
-            const uint8_t *out_tile = p.out + p.out_base + n_base;
-            // G M tiles at a time: the 16 bytes of constants a column needs are loaded from shared memory once and serve G
-            // outputs (those loads are what saturates first in the one-tile form: two LSU wavefronts per output and warp).
-            constexpr bool kPlainPack = MODE == kModeReluSat;      // packed bytes are final: no lower clamp to add, no sign flip
-            auto multi_tiles = [&](auto gtag) {
-                constexpr int G = decltype(gtag)::value;
-                for (int j0 = 0; j0 < nsub; j0 += G, ++wrot) {
-                    const int gn = min(G, nsub - j0);
-                    const int m0 = (tg * p.group + j0) * kBM;
-                    // Decided alike by every epilogue warp: all G tiles lie inside the matrix and every chunk is 16 real columns
-                    // (no conditions in the loop); then, where rows and chunk pairs start on 32-byte boundaries, a thread's two
-                    // chunks leave as one 32-byte store (a whole sector, half as many requests to the L2 as 16-byte stores).
-                    const bool full = gn == G && m0 + G * kBM <= p.M && n_cols == (cps << 4);
-                    const bool wide = full && wide_ok;
-                    int wfirst = cgrp + static_cast<int>(wrot % kColGroups);      // 32-column chunk wc belongs to group (wc - wrot) mod kColGroups
-                    if (wfirst >= kColGroups) wfirst -= kColGroups;
-                    if (wide ? wfirst < (cps >> 1) : first < cps) {
-                        uint8_t *orow[G];
-                        bool live[G];
-                        int32_t asum_term[G];
-                        uint32_t t_tile[G];
+            t.n_left = min(p.bn_data, p.N - n_base);
+            for (int j = 0; j < nsub && !(ENN_DBG_MODE(p) & 2); ++j) {
+                int first = cols_shared ? (cgrp + turn) % kColGroups : cgrp;
+                turn = (turn + ng) % kColGroups;
+                if (first >= ng) continue;
+                const int tm = TWO ? tg * 2 + static_cast<int>(rank) : tg * p.group + j;
+                const int m0 = tm * kBM + q * 32;
+                t.live = 0;
+                if (p.qh == 1) {
+                    uint8_t *r0 = p.out + p.out_base + n_base + static_cast<int64_t>(m0 + (lane >> 2)) * p.out_sx;
 #pragma unroll
-                        for (int i = 0; i < G; ++i) {
-                            const int m = m0 + i * kBM + row_in_tile;
-                            live[i] = i < gn && m < p.M;
-                            orow[i] = const_cast<uint8_t *>(out_tile) + static_cast<int64_t>(live[i] ? m : 0) * p.out_sx;
-                            // a slot the unit does not have re-reads the first one (unused)
-                            t_tile[i] = t_row + (j0 + i < p.group ? j0 + i : j0) * p.bn_rows;
-                            asum_term[i] = 0;
-                            if (ASUM) {
-                                uint32_t rs;
-                                tmem_ld_x1(t_tile[i] + p.bn_data, rs);       // warp-collective
-                                tmem_ld_wait();
-                                asum_term[i] = p.zw_eff * static_cast<int32_t>(rs);
-                            }
-                        }
-                        // One chunk loop.  STORE 0: 16-byte global stores under the per-row and per-chunk conditions; 1: stores
-                        // without conditions.  CW: 16-column chunks per step (2 with STORE 1 only).
-                        auto chunks = [&](auto storetag, auto widthtag) {
-                            constexpr int STORE = decltype(storetag)::value;
-                            constexpr int CW = decltype(widthtag)::value;
-                            for (int c0 = CW == 2 ? wfirst << 5 : first << 4; c0 < (cps << 4); c0 += kColGroups * 16 * CW) {
-                                const uint32_t lc = (CW == 2 || cols_shared) ? lc_shared + c0 * 16 : lc_private;
-                                const uint8_t *lcp = s_cols_sp + (lc - s_cols_u32);
-                                if (CW == 1) lc_private += 256;
-                                uint32_t w[G][4 * CW];
-                                // Accumulators: one 16-column load per tile while the registers allow it (G <= 2), else 8 columns.
-                                constexpr int LW = G <= 2 ? 16 : 8;
-#pragma unroll
-                                for (int part = 0; part < 16 * CW / LW; ++part) {
-                                    uint32_t r[G][LW];
-#pragma unroll
-                                    for (int i = 0; i < G; ++i) {      // warp-collective
-                                        if constexpr (LW == 16) tmem_ld_x16(t_tile[i] + c0 + 16 * part, r[i]);
-                                        else tmem_ld_x8(t_tile[i] + c0 + 8 * part, r[i]);
-                                    }
-                                    tmem_ld_wait();
-#pragma unroll
-                                    for (int jj = 0; jj < LW / 4; ++jj) {
-                                        int32_t y[G][4];
-#pragma unroll
-                                        for (int b = 0; b < 4; ++b) {
-                                            ColRegs cv;
-                                            ld_col_shared<MODE>(lcp + (part * LW + jj * 4 + b) * 16, cv);
-#pragma unroll
-                                            for (int i = 0; i < G; ++i) {
-                                                int32_t acc = static_cast<int32_t>(r[i][jj * 4 + b]);
-                                                if (ASUM) acc -= asum_term[i];
-                                                y[i][b] = tc_requant<MODE>(acc, cv, hi_clamp, p.out_zp, p.act_min, p.act_max);
-                                            }
-                                        }
-#pragma unroll
-                                        for (int i = 0; i < G; ++i) {
-                                            const uint32_t hi = pack_sat_u8_tc(y[i][3], y[i][2], 0);
-                                            const uint32_t pk = pack_sat_u8_tc(y[i][1], y[i][0], hi);
-                                            w[i][part * (LW / 4) + jj] = kPlainPack ? pk : ((pk + lo_word) ^ sign_word);
-                                        }
-                                    }
-                                }
-                                if constexpr (FADD) {
-#pragma unroll
-                                    for (int i = 0; i < G; ++i)
-                                        if (STORE == 1 || (live[i] && c0 < n_cols)) {
-#pragma unroll
-                                            for (int h = 0; h < CW; ++h) {
-                                                uint32_t (&wq)[4] = *reinterpret_cast<uint32_t (*)[4]>(&w[i][4 * h]);
-                                                fadd_chunk(wq, orow[i] + c0 + 16 * h + res_delta, fadd);
-                                            }
-                                        }
-                                }
-                                if constexpr (CW == 2) {
-#pragma unroll
-                                    for (int i = 0; i < G; ++i)
-                                        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(orow[i] + c0), "r"(w[i][0]), "r"(w[i][1]),
-                                                     "r"(w[i][2]), "r"(w[i][3]), "r"(w[i][4]), "r"(w[i][5]), "r"(w[i][6]), "r"(w[i][7])
-                                                     : "memory");
-                                } else if (STORE == 1 || c0 < n_cols) {
-#pragma unroll
-                                    for (int i = 0; i < G; ++i)
-                                        if (STORE == 1 || live[i]) *reinterpret_cast<uint4 *>(orow[i] + c0) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
-                                }
-                            }
-                        };
-                        constexpr std::integral_constant<int, 1> one{};
-                        if (wide) chunks(one, std::integral_constant<int, 2>{});
-                        else if (full) chunks(one, one);
-                        else chunks(std::integral_constant<int, 0>{}, one);
+                    for (int h = 0; h < 4; ++h) {
+                        t.live |= m0 + (lane >> 2) + 8 * h < p.M ? 1u << h : 0u;
+                        t.row[h] = r0 + 8 * h * p.out_sx;
                     }
-                    first -= cps_mod;
-                    if (first < 0) first += kColGroups;
-                }
-            };
-            if (epi_g == 4) multi_tiles(std::integral_constant<int, 4>{});
-            else if (epi_g == 2) multi_tiles(std::integral_constant<int, 2>{});
-            for (int j = 0; j < nsub && epi_g == 0 && !(ENN_DBG_MODE(p) & 2); ++j) {
-                if (first < cps) {
-                    const int tm = TWO ? tg * 2 + static_cast<int>(rank) : tg * p.group + j;
-                    const int m = tm * kBM + row_in_tile;
-                    bool row_ok = m < p.M;
-                    uint8_t *orow;
-                    if (p.taps > 0) {
-                        const int per_img = p.conv_ty * p.conv_tx;
-                        const int img = tm / per_img, rem = tm - img * per_img;
-                        const int ty = rem / p.conv_tx, tx = rem - ty * p.conv_tx;
-                        const int qy = ty * p.conv_ht + patch_y, qx = tx * p.conv_wt + patch_x;
-                        row_ok = patch_y < p.conv_ht && qy < p.qh && qx < p.qw;
-                        orow = const_cast<uint8_t *>(out_tile) + img * p.out_sn + (row_ok ? qy : 0) * p.out_sy + (row_ok ? qx : 0) * p.out_sx;
-                    } else if (p.qh == 1) {
-                        orow = const_cast<uint8_t *>(out_tile) + static_cast<int64_t>(row_ok ? m : 0) * p.out_sx;
-                    } else {
-                        const int mq = row_ok ? m : 0;
-                        const int img = mq / (p.qh * p.qw), rem = mq - img * (p.qh * p.qw);
+                } else {        // rows of an output grid: lane l works out row l, a thread takes its four rows from the lanes
+                    const int m = m0 + lane;
+                    int64_t off = -1;
+                    if (m < p.M) {
+                        const int img = m / (p.qh * p.qw), rem = m - img * (p.qh * p.qw);
                         const int qy = rem / p.qw, qx = rem - qy * p.qw;
-                        orow = const_cast<uint8_t *>(out_tile) + img * p.out_sn + qy * p.out_sy + qx * p.out_sx;
+                        off = p.out_base + n_base + img * p.out_sn + qy * p.out_sy + qx * p.out_sx;
                     }
-                    const uint32_t t_tile = t_row + j * p.bn_rows;
-                    int32_t asum_term = 0;
-                    if (ASUM) {
-                        uint32_t rs;
-                        tmem_ld_x1(t_tile + p.bn_data, rs);       // warp-collective
-                        tmem_ld_wait();
-                        asum_term = p.zw_eff * static_cast<int32_t>(rs);
-                    }
-                    // Requantises the 8 accumulators of one half chunk into two packed words.
-                    auto half_chunk = [&](const uint32_t (&r)[8], uint32_t lc_half, uint32_t &w0, uint32_t &w1) {
 #pragma unroll
-                        for (int jj = 0; jj < 2; ++jj) {
-                            int32_t y[4];
-#pragma unroll
-                            for (int b = 0; b < 4; ++b) {
-                                ColRegs cv;
-                                ld_col_shared<MODE>(s_cols_sp + (lc_half - s_cols_u32) + (jj * 4 + b) * 16, cv);
-                                int32_t acc = static_cast<int32_t>(r[jj * 4 + b]);
-                                if (ASUM) acc -= asum_term;
-                                y[b] = tc_requant<MODE>(acc, cv, hi_clamp, p.out_zp, p.act_min, p.act_max);
-                            }
-                            const uint32_t hi = pack_sat_u8_tc(y[3], y[2], 0);
-                            const uint32_t pk = pack_sat_u8_tc(y[1], y[0], hi);
-                            (jj == 0 ? w0 : w1) = kPlainPack ? pk : ((pk + lo_word) ^ sign_word);
-                        }
-                    };
-                    if (whole_rows && n_cols == (cps << 4) && m + (kBM - 1 - row_in_tile) < p.M) {
-                        // The usual case, decided per warp: the M tile lies inside the matrix, every chunk is 16 real columns and
-                        // one aligned 16-byte store.  No per-thread conditions, so nothing here diverges.
-                        for (int c0 = first << 4; c0 < (cps << 4); c0 += kColGroups * 16, lc_private += 256) {
-                            const uint32_t lc = cols_shared ? lc_shared + c0 * 16 : lc_private;
-                            uint32_t w[4];
-#pragma unroll
-                            for (int half = 0; half < 2; ++half) {
-                                uint32_t r[8];
-                                tmem_ld_x8(t_tile + c0 + 8 * half, r);      // warp-collective
-                                tmem_ld_wait();
-                                half_chunk(r, lc + half * 128, w[half * 2], w[half * 2 + 1]);
-                            }
-                            if constexpr (FADD) fadd_chunk(w, orow + c0 + res_delta, fadd);
-                            *reinterpret_cast<uint4 *>(orow + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-                    for (int c0 = first << 4; c0 < (cps << 4); c0 += kColGroups * 16, lc_private += 256) {
-                        const uint32_t lc = cols_shared ? lc_shared + c0 * 16 : lc_private;
-                        // two 8-column loads per chunk: half the accumulator registers live at a time
-                        uint32_t w[4];
-#pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            uint32_t r[8];
-                            tmem_ld_x8(t_tile + c0 + 8 * half, r);      // warp-collective
-                            tmem_ld_wait();
-                            if (row_ok && c0 < n_cols) half_chunk(r, lc + half * 128, w[half * 2], w[half * 2 + 1]);
-                        }
-                        if (row_ok && c0 < n_cols) {
-                            if constexpr (FADD) fadd_chunk(w, orow + c0 + res_delta, fadd);      // fused operators have 16-byte rows (plan)
-                            if (ENN_DBG_MODE(p) & 4) {
-                                // development switch: no stores (isolates the store path; only one lane keeps the values alive)
-                                if ((w[0] ^ w[1] ^ w[2] ^ w[3]) == 0x12345678u && lane == 33) orow[0] = 1;
-                            } else if (st_fast) {
-                                *reinterpret_cast<uint4 *>(orow + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                            } else {
-                                const int left = n_cols - c0;
-                                if (st_align == 16 && left >= 16) {
-                                    *reinterpret_cast<uint4 *>(orow + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                                } else if (st_align >= 8 && left >= 8) {
-                                    *reinterpret_cast<uint2 *>(orow + c0) = make_uint2(w[0], w[1]);
-                                    if (left >= 16) {
-                                        *reinterpret_cast<uint2 *>(orow + c0 + 8) = make_uint2(w[2], w[3]);
-                                    } else {
-#pragma unroll
-                                        for (int b = 8; b < 16; ++b)
-                                            if (b < left) orow[c0 + b] = static_cast<uint8_t>(w[b >> 2] >> (8 * (b & 3)));
-                                    }
-                                } else {
-#pragma unroll
-                                    for (int b = 0; b < 16; ++b)
-                                        if (b < left) orow[c0 + b] = static_cast<uint8_t>(w[b >> 2] >> (8 * (b & 3)));
-                                }
-                            }
-                        }
+                    for (int h = 0; h < 4; ++h) {
+                        const int64_t o = __shfl_sync(0xffffffffu, off, (lane >> 2) + 8 * h);
+                        t.live |= o >= 0 ? 1u << h : 0u;
+                        t.row[h] = p.out + o;
                     }
                 }
-                }
-                // first chunk of this warp in the next M tile
-                first -= cps_mod;
-                if (first < 0) first += kColGroups;
+                const uint32_t t_row = t_buf + j * p.bn_rows;
+                if (ASUM) epi_asum(t_row, p.bn_data, p.zw_eff, lane, t.asum);
+                const uint8_t *shared = s_cols_sp + tn * p.bn_rows * 16;
+                epi_tile<MODE, ASUM, FADD>(t_row, first, kColGroups, p.bn_data, t, lane, e, [&](int c0) {
+                    return cols_shared ? shared : s_cols_sp + priv + (c0 / 32 / kColGroups) * 512 - c0 * 16;
+                });
             }
             tc_fence_before();
             __syncwarp();
@@ -908,7 +642,7 @@ gemv_kernel(const uint8_t *__restrict__ a, const int8_t *__restrict__ w, const C
     const int n = blockIdx.x * kGemvWarps + warp;
     const bool active = n < N;
     const int tn = active ? n / bn_data : 0, r = active ? n - tn * bn_data : 0;
-    const uint4 *wrow = reinterpret_cast<const uint4 *>(w + (static_cast<size_t>(tn) * bn_rows + r) * k_pad);
+    const uint4 *wrow = reinterpret_cast<const uint4 *>(w + (static_cast<size_t>(tn) * bn_rows + tile_row(r, bn_data)) * k_pad);
     // The weights are the operator's constants: the first kGemvAhead 512-byte pieces of this warp's column (all of it up
     // to K = 4096) are requested before the wait on the kernel that produces the activations and before the
     // activations are staged, so that the whole weight stream is in flight from the first instruction on.
@@ -957,7 +691,7 @@ gemv_kernel(const uint8_t *__restrict__ a, const int8_t *__restrict__ w, const C
             asum[m] += __shfl_xor_sync(0xffffffffu, asum[m], off);
         }
     if (lane == 0) {
-        const ColParam c = cols[static_cast<size_t>(tn) * bn_rows + r];
+        const ColParam c = cols[static_cast<size_t>(tn) * bn_rows + tile_slot(r, bn_data)];
         const int4 cv = make_int4(c.mult, c.addend, c.esh, c.bias);
 #pragma unroll
         for (int m = 0; m < M; ++m) {
@@ -1067,29 +801,6 @@ __global__ void im2col_kernel(Im2colGeom g, const uint8_t *__restrict__ in, uint
     reinterpret_cast<uint4 *>(out)[t] = v;
 }
 
-// ------------------------------------------------------------------------------------------------------
-// Host side
-// ------------------------------------------------------------------------------------------------------
-// Copies an NHWC tensor into a larger one with `lo_y` / `lo_x` extra rows / columns before and extra ones after, filled
-// with the input zero point: what the reference's pad kernels produce (PadConvertKernels.cpp:241-373), so that the
-// tap boxes of the implicit convolution never meet a border.  One thread writes 16 bytes (C % 16 == 0).
-__global__ void pad_nhwc_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int n, int h, int w, int c, int hp, int wp, int lo_y,
-                                int lo_x, uint32_t fill, int64_t total16) {
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= total16) return;
-    const int c16 = c >> 4;
-    const int cc = static_cast<int>(t % c16);
-    int64_t r = t / c16;
-    const int x = static_cast<int>(r % wp);
-    r /= wp;
-    const int y = static_cast<int>(r % hp);
-    const int img = static_cast<int>(r / hp);
-    const int iy = y - lo_y, ix = x - lo_x;
-    uint4 v = make_uint4(fill, fill, fill, fill);
-    if (iy >= 0 && iy < h && ix >= 0 && ix < w) v = __ldg(reinterpret_cast<const uint4 *>(in + ((static_cast<int64_t>(img) * h + iy) * w + ix) * c) + cc);
-    reinterpret_cast<uint4 *>(out)[t] = v;
-}
-
 void launch_im2col(const Im2colGeom &ig, const void *in, uint8_t *dst, int64_t total16, unsigned blocks, cudaStream_t s) {
     const uint8_t *src = static_cast<const uint8_t *>(in);
     const uintptr_t a = reinterpret_cast<uintptr_t>(in);
@@ -1148,8 +859,8 @@ __global__ void __launch_bounds__(256) conv3x3c3_kernel(Conv3x3c3Params g, const
     uint4 *s_w = smem_q;                 // [N][2] : 32 weight bytes per output channel (27 real, 5 zero)
     uint4 *s_c = smem_q + 2 * g.N;       // [N]    : epilogue constants
     for (int i = threadIdx.x; i < 2 * g.N; i += blockDim.x)
-        s_w[i] = *reinterpret_cast<const uint4 *>(wq + static_cast<size_t>(i >> 1) * g.k_pad + (i & 1) * 16);
-    for (int i = threadIdx.x; i < g.N; i += blockDim.x) s_c[i] = *reinterpret_cast<const uint4 *>(cols + i);
+        s_w[i] = *reinterpret_cast<const uint4 *>(wq + static_cast<size_t>(tile_row(i >> 1, g.N)) * g.k_pad + (i & 1) * 16);
+    for (int i = threadIdx.x; i < g.N; i += blockDim.x) s_c[i] = *reinterpret_cast<const uint4 *>(cols + tile_slot(i, g.N));
     __syncthreads();
     pdl_wait();         // weights and constants above belong to the plan; the image may come from the kernel before
     pdl_trigger();
@@ -1279,12 +990,6 @@ struct TcGemm {
     bool gather = false;               // A is gathered into scratch by im2col first
     bool first_layer = false;          // 3x3 taps over 3 channels: conv3x3c3_kernel instead of gather + GEMM
     bool use_gemv = false;             // M <= 8 read in place: weight-streaming GEMV instead of the tensor-core kernel
-    // Implicit convolution (stride-1 taps read as TMA boxes, no gathered matrix): the source is either the caller's
-    // tensor (input zero point 0: the zero OOB fill is already right) or a zero-point padded copy in scratch.
-    bool implicit = false;
-    bool padded = false;
-    bool runs_pad = false;             // this GEMM launches the pad pass (the first padded GEMM of the operator)
-    int32_t pad_lo_y = 0, pad_lo_x = 0, hp = 0, wp = 0;
     Im2colGeom ig{};
     CUtensorMap map_a_static{};        // A map over the library's static scratch array (no-allocation entry point)
     const void *map_a_static_ptr = nullptr;
@@ -1295,7 +1000,6 @@ struct TcPlan {
     void *scratch = nullptr;           // im2col matrix, shared by the GEMMs of the op (they run in stream order)
     size_t scratch_bytes = 0;
     std::unique_ptr<GcPlan> gc;        // gather convolution (gconv.cu): replaces the list of GEMMs
-    bool fan_out = false;              // the GEMMs are independent (deconvolution classes): run them side by side
     int32_t *err_host = nullptr;       // pinned + mapped
     int32_t *err_dev = nullptr;
     bool starve_next = false;          // the next execute runs the bounded-wait self-test (tc_test_starve_next)
@@ -1303,31 +1007,17 @@ struct TcPlan {
     const uint8_t *residual = nullptr; // the add's other input for the next execute
 };
 
-// NHWC activation tensor {C, W, H, N} with a box of {span channels, box_w, box_h, 1}.
-bool encode_nhwc(enn_b200_context *ctx, CUtensorMap *map, const void *base, uint64_t c, uint64_t w, uint64_t h, uint64_t n, uint32_t span,
-                 uint32_t box_w, uint32_t box_h) {
-    EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled);
-    if (!fn) return false;
-    cuuint64_t dims[4] = {c, w, h, n};
-    cuuint64_t strides[3] = {c, w * c, h * w * c};
-    cuuint32_t box[4] = {span, box_w, box_h, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle_of(span), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
 // Builds one GEMM: packs B, folds zero points into the bias, derives the epilogue constants, sizes the launch.
 // weight(n, k) returns the raw weight byte of output column n at reduction index k (k < K).
 template <typename WeightFn>
 int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh, int32_t M, int32_t N, int32_t K, WeightFn weight,
-                   TcGemm *gm, uint32_t implicit_span = 0, bool want_resident = false) {
+                   TcGemm *gm, bool want_resident = false) {
     TcParams &p = gm->prm;
     p.M = M; p.N = N; p.K = K;
     // K bytes per k-block.  Implicit convolutions bring theirs (the channel chunk); plain GEMMs with a short K use 32-
     // or 64-byte rows, so that the TMA does not spend its time zero-filling 128-byte rows that are mostly padding.
-    uint32_t span = implicit_span ? implicit_span : (K <= 32 ? 32u : (K <= 64 ? 64u : static_cast<uint32_t>(kBK)));
-    if (ctx->opt("no_narrow_span") && !implicit_span) span = kBK;
+    uint32_t span = K <= 32 ? 32u : (K <= 64 ? 64u : static_cast<uint32_t>(kBK));
+    if (ctx->opt("no_narrow_span")) span = kBK;
     p.span = static_cast<int32_t>(span);
     const int32_t zw_eff = g.w_signed ? g.w_zp : g.w_zp - 128;   // weights as signed bytes: int8 stays, u8 becomes w - 128
     p.zw_eff = zw_eff;
@@ -1343,7 +1033,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     // a column's constants serves two outputs (28 x 28 x 32 -> 192 at 256 images: 24.2 -> 21.1 us; 14 x 14 x 96 -> 576:
     // 21.7 -> 19.9 us; 56 x 56 x 24 -> 144 in its four-pixel packing, 576 columns: 73.8 -> 65.4 us; 384 and 960 columns:
     // no change).  Not with the extra column of the activation sums, which would leave room for one M tile only.
-    if (!implicit_span && !ctx->has_opt("tc_bn") && !ctx->opt("no_narrow_n") && K <= static_cast<int32_t>(span) && N > 128 && extra == 0 &&
+    if (!ctx->has_opt("tc_bn") && !ctx->opt("no_narrow_n") && K <= static_cast<int32_t>(span) && N > 128 && extra == 0 &&
         M > kGemvMaxM && max_data > 128)
         max_data = 128;
     // N tiling: as few tiles as possible, but split further while the grid would leave SMs idle.
@@ -1367,7 +1057,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     // CTA pairs (cta_group::2): two SMs share one 256-row tile and every B byte is fetched once per pair.  Used for plain
     // GEMMs with several waves of 256-wide tiles, long K and large operands ((M+N) K >= 32 MB): 8192^3 runs 7 % faster
     // than on the one-CTA kernel, 4096^3 6 % (51.6 against 54.7 us).  Option tc_pair = 0 / 1 overrides the size rule.
-    const bool pair_ok = span == kBK && !implicit_span && p.tiles_m >= 2 && (K + kBK - 1) / kBK >= 8 && bn_data >= 128 &&
+    const bool pair_ok = span == kBK && p.tiles_m >= 2 && (K + kBK - 1) / kBK >= 8 && bn_data >= 128 &&
                          static_cast<int64_t>(p.tiles_m) * tiles_n >= 2ll * ctx->sm_count;
     bool two = pair_ok && (static_cast<int64_t>(M) + N) * K >= (32ll << 20);
     int32_t forced_rows = 0;
@@ -1413,7 +1103,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     std::vector<ColumnFold> folds(N);
     for (int32_t n = 0; n < N; ++n) {
         const int32_t tn = n / bn_data, r = n % bn_data;
-        int8_t *dst = wb.data() + (static_cast<size_t>(tn) * p.bn_rows + r) * k_pad;
+        int8_t *dst = wb.data() + (static_cast<size_t>(tn) * p.bn_rows + tile_row(r, bn_data)) * k_pad;
         int64_t wsum = 0, wabs = 0;
         for (int32_t k = 0; k < K; ++k) {
             const uint8_t raw = weight(n, k);
@@ -1427,7 +1117,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     p.mode = column_mode(ctx, g, qh, folds, N, M > kGemvMaxM);
     p.sat_plain = column_sat_plain(ctx, g, p.mode);
     for (int32_t n = 0; n < N; ++n)
-        if (!column_constants(g, p.mode, qh.mult[n], qh.shift[n], folds[n], &cols[static_cast<size_t>(n / bn_data) * p.bn_rows + n % bn_data])) p.mode = kModeGeneral;
+        if (!column_constants(g, p.mode, qh.mult[n], qh.shift[n], folds[n], &cols[static_cast<size_t>(n / bn_data) * p.bn_rows + tile_slot(n % bn_data, bn_data)])) p.mode = kModeGeneral;
     if (p.need_asum)
         for (int32_t tn = 0; tn < tiles_n; ++tn) {
             int8_t *dst = wb.data() + (static_cast<size_t>(tn) * p.bn_rows + bn_data) * k_pad;
@@ -1450,14 +1140,14 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     // copy per ~420 cycles and a tile needs one A and one B copy per k-block): when the weights of the only N tile fit,
     // they are loaded once per CTA and stay resident, the stages hold A only, and the producer issues half as many copies.
     const size_t b_tile = (static_cast<size_t>(p.bn_rows) * span + 1023) & ~static_cast<size_t>(1023);
-    p.b_res = ((implicit_span != 0 || p.bn_rows <= 64 || want_resident || (p.k_blocks == 1 && !ctx->opt("no_bres_k1"))) && !p.two && tiles_n == 1 && M > kGemvMaxM && b_tile * p.k_blocks <= (want_resident ? kWidePackWeightBytes : 72 * 1024) &&
+    p.b_res = ((p.bn_rows <= 64 || want_resident || (p.k_blocks == 1 && !ctx->opt("no_bres_k1"))) && !p.two && tiles_n == 1 && M > kGemvMaxM && b_tile * p.k_blocks <= (want_resident ? kWidePackWeightBytes : 72 * 1024) &&
                !ctx->opt("no_bres")) ? 1 : 0;
     const size_t kb_bytes = p.b_res ? static_cast<size_t>(kBM) * span : (static_cast<size_t>(kBM) + (p.two ? p.bn_rows / 2 : p.bn_rows)) * span;
     p.kpack = static_cast<int32_t>((32 * 1024) / kb_bytes);
     if (p.kpack < 1 || p.two) p.kpack = 1;
     if (p.kpack > p.k_blocks) p.kpack = p.k_blocks;
     if (p.kpack > 8) p.kpack = 8;
-    const size_t fixed = static_cast<size_t>(kEpiWarps) * kChunksPerWarp * 16 * sizeof(ColParam) + 1024 + 1024;   // column constants, barriers, slack
+    const size_t fixed = static_cast<size_t>(kColEntries) * sizeof(ColParam) + 1024 + 1024;   // column constants, barriers, slack
     const size_t resident = p.b_res ? b_tile * p.k_blocks : 0;
     const size_t stage_bytes = kb_bytes * p.kpack;
     int stages = static_cast<int>((227 * 1024 - fixed - resident) / stage_bytes);
@@ -1472,9 +1162,6 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     // One thread cannot issue both operands of every k-block fast enough for a long MMA-bound k loop; short, epilogue-
     // bound problems are better off without the extra warp.
     gm->threads = (p.kpack == 1 && p.k_blocks >= 8) ? kThreads : kThreadsOneProducer;
-    p.epi_g = p.two ? 1 : (p.group >= 4 ? 4 : (p.group >= 2 ? 2 : 1));
-    p.no_wide_store = ctx->opt("no_wide_store") ? 1 : 0;
-    if (ctx->has_opt("epi_g")) { const int ev = ctx->opt("epi_g"); p.epi_g = ev == 4 || ev == 2 ? (ev <= p.group ? ev : p.epi_g) : 1; }   // tuning override
     return ENN_B200_SUCCESS;
 }
 
@@ -1574,7 +1261,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
             tab[static_cast<size_t>(p.cls[i].tab0 + k / p.gran)] = make_int2(static_cast<int>(off), (dy << 16) | (dx & 0xffff));
         }
         for (int32_t n = 0; n < N; ++n) {
-            int8_t *dst = wb.data() + ((static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + n % p.bn_data) * k_pad;
+            int8_t *dst = wb.data() + ((static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + tile_row(n % p.bn_data, p.bn_data)) * k_pad;
             int64_t wsum = 0, wabs = 0;
             for (int32_t k = 0; k < K; ++k) {
                 const uint8_t raw = weight(i, n, k);
@@ -1597,7 +1284,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     for (int32_t i = 0; i < nc; ++i)
         for (int32_t n = 0; n < N; ++n)
             if (!column_constants(g, p.mode, qh.mult[n], qh.shift[n], folds[static_cast<size_t>(i) * N + n],
-                                  &cols[(static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + n % p.bn_data]))
+                                  &cols[(static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + tile_slot(n % p.bn_data, p.bn_data)]))
                 p.mode = kModeGeneral;
     cudaError_t e;
     if ((e = cudaMalloc(&gc->w_dev, wb.size())) != cudaSuccess || (e = cudaMalloc(&gc->cols_dev, cols.size() * sizeof(ColParam))) != cudaSuccess ||
@@ -1761,63 +1448,21 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
     const uint32_t fill = (static_cast<uint32_t>(g.in_zp) & 0xff) * 0x01010101u;
     int32_t st = ENN_B200_SUCCESS;
 
-    // Decides how a GEMM whose A operand is described by `ig` (grid oh x ow per image, taps kh x kw) gets that operand and
-    // builds it: implicit convolution (stride-1 taps, Cin % 32 == 0) or gathered matrix.  `weight(n, k)` uses k = tap * cin + c.
+    // A GEMM whose A operand is gathered into scratch first (im2col_kernel): what the gather convolution does not cover, i.e.
+    // channel counts that are no multiple of 4.  `weight(n, k)` uses k = tap * cin + c.
     auto make_conv_gemm = [&](TcGemm &gm, const Im2colGeom &ig, auto weight) -> int32_t {
         const int32_t K = ig.kh * ig.kw * cin;
-        const int32_t taps = ig.kh * ig.kw;
-        uint32_t span = 0;
-        if (ig.sy == 1 && ig.sx == 1 && (cin & 31) == 0 && taps <= 64 && !ctx->opt("no_implicit"))
-            span = (cin % 128 == 0) ? 128 : ((cin % 64 == 0) ? 64 : 32);
         const int64_t M64 = static_cast<int64_t>(ig.n) * ig.oh * ig.ow;
         if (M64 <= 0 || M64 > INT32_MAX) return ENN_B200_INVALID_PARAMS;
         gm.ig = ig;
-        if (!span) {
-            int32_t st2 = build_gemm(ctx, g, qh, static_cast<int32_t>(M64), N, K, weight, &gm);
-            if (st2 != ENN_B200_SUCCESS) return st2;
-            gm.gather = true;
-            gm.ig.K = K; gm.ig.Kp = (K + 15) & ~15;
-            gm.first_layer = ig.kh == 3 && ig.kw == 3 && cin == 3 && ig.dy == 1 && ig.dx == 1 && (N & 15) == 0 && gm.prm.tiles_n == 1 &&
-                             M64 >= 4096 && !ctx->opt("no_first_layer");
-            const size_t need = static_cast<size_t>(M64) * gm.ig.Kp;
-            if (need > plan->scratch_bytes) plan->scratch_bytes = need;
-            return ENN_B200_SUCCESS;
-        }
-        // patch of the output grid per M tile: as wide as the grid allows, rows to fill 128 accumulator rows
-        const int32_t wt = ig.ow < kBM ? ig.ow : kBM;
-        int32_t ht = kBM / wt;
-        if (ht > ig.oh) ht = ig.oh;
-        const int32_t tx = (ig.ow + wt - 1) / wt, ty = (ig.oh + ht - 1) / ht;
-        const int64_t tiles = static_cast<int64_t>(ig.n) * tx * ty;
-        if (tiles * kBM > INT32_MAX) return ENN_B200_INVALID_PARAMS;
-        int32_t st2 = build_gemm(ctx, g, qh, static_cast<int32_t>(tiles * kBM), N, K, weight, &gm, span);
+        const int32_t st2 = build_gemm(ctx, g, qh, static_cast<int32_t>(M64), N, K, weight, &gm);
         if (st2 != ENN_B200_SUCCESS) return st2;
-        TcParams &p = gm.prm;
-        p.taps = taps; p.cchunks = cin / static_cast<int32_t>(span); p.span = static_cast<int32_t>(span);
-        p.conv_ht = ht; p.conv_wt = wt; p.conv_ty = ty; p.conv_tx = tx;
-        int32_t min_dy = 0, max_dy = 0, min_dx = 0, max_dx = 0;
-        for (int32_t ky = 0; ky < ig.kh; ++ky)
-            for (int32_t kx = 0; kx < ig.kw; ++kx) {
-                const int32_t dy = ky * ig.dy + ig.y0, dx = kx * ig.dx + ig.x0;
-                min_dy = dy < min_dy ? dy : min_dy; max_dy = dy > max_dy ? dy : max_dy;
-                min_dx = dx < min_dx ? dx : min_dx; max_dx = dx > max_dx ? dx : max_dx;
-            }
-        gm.implicit = true;
-        gm.padded = g.in_zp != 0;            // zero OOB fill already equals the zero point otherwise
-        gm.pad_lo_y = gm.padded ? -min_dy : 0;
-        gm.pad_lo_x = gm.padded ? -min_dx : 0;
-        const int32_t hi_y = ig.oh - 1 + max_dy - (ig.h - 1), hi_x = ig.ow - 1 + max_dx - (ig.w - 1);
-        gm.hp = gm.padded ? gm.pad_lo_y + ig.h + (hi_y > 0 ? hi_y : 0) : ig.h;
-        gm.wp = gm.padded ? gm.pad_lo_x + ig.w + (hi_x > 0 ? hi_x : 0) : ig.w;
-        for (int32_t ky = 0; ky < ig.kh; ++ky)
-            for (int32_t kx = 0; kx < ig.kw; ++kx) {
-                p.tap_dy[ky * ig.kw + kx] = static_cast<int16_t>(ky * ig.dy + ig.y0 + gm.pad_lo_y);
-                p.tap_dx[ky * ig.kw + kx] = static_cast<int16_t>(kx * ig.dx + ig.x0 + gm.pad_lo_x);
-            }
-        if (gm.padded) {
-            const size_t need = static_cast<size_t>(ig.n) * gm.hp * gm.wp * cin;
-            if (need > plan->scratch_bytes) plan->scratch_bytes = need;
-        }
+        gm.gather = true;
+        gm.ig.K = K; gm.ig.Kp = (K + 15) & ~15;
+        gm.first_layer = ig.kh == 3 && ig.kw == 3 && cin == 3 && ig.dy == 1 && ig.dx == 1 && (N & 15) == 0 && gm.prm.tiles_n == 1 &&
+                         M64 >= 4096 && !ctx->opt("no_first_layer");
+        const size_t need = static_cast<size_t>(M64) * gm.ig.Kp;
+        if (need > plan->scratch_bytes) plan->scratch_bytes = need;
         return ENN_B200_SUCCESS;
     };
 
@@ -1914,7 +1559,7 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             auto packed_weight = [&](int32_t n, int32_t k) -> uint8_t {
                 return n / N == k / K ? weight(n % N, k % K) : zero_raw;
             };
-            st = build_gemm(ctx, g, qp, static_cast<int32_t>(M64 / pack), pack * N, pack * K, packed_weight, &gm, 0, wide_pack);
+            st = build_gemm(ctx, g, qp, static_cast<int32_t>(M64 / pack), pack * N, pack * K, packed_weight, &gm, wide_pack);
             if (st != ENN_B200_SUCCESS) return bail(st);
             gm.prm.qh = 1; gm.prm.qw = static_cast<int32_t>(M64 / pack);
             gm.prm.out_base = 0; gm.prm.out_sn = 0; gm.prm.out_sy = 0; gm.prm.out_sx = pack * N;
@@ -1939,16 +1584,8 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             }
             st = make_conv_gemm(gm, ig, weight);
             if (st != ENN_B200_SUCCESS) return bail(st);
-            if (gm.implicit) {
-                gm.prm.qh = g.oh; gm.prm.qw = g.ow;
-                gm.prm.out_base = 0;
-                gm.prm.out_sn = static_cast<int64_t>(g.oh) * g.ow * N;
-                gm.prm.out_sy = static_cast<int64_t>(g.ow) * N;
-                gm.prm.out_sx = N;
-            } else {
-                gm.prm.qh = 1; gm.prm.qw = static_cast<int32_t>(M64);
-                gm.prm.out_base = 0; gm.prm.out_sn = 0; gm.prm.out_sy = 0; gm.prm.out_sx = N;
-                }
+            gm.prm.qh = 1; gm.prm.qw = static_cast<int32_t>(M64);
+            gm.prm.out_base = 0; gm.prm.out_sn = 0; gm.prm.out_sy = 0; gm.prm.out_sx = N;
         }
     } else {
         // Transposed convolution (DeconvolutionKernels.cpp:24-198) split by output parity: outputs with
@@ -2023,48 +1660,8 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             }
         }
         if (plan->gemms.empty()) return bail(ENN_B200_INVALID_PARAMS);
-        // The classes write disjoint outputs and only read the (padded) input: give each a share of the SMs and launch
-        // them on side streams, so that their launch and pipeline latencies overlap instead of adding up.
-        const int ncls = static_cast<int>(plan->gemms.size());
-        bool all_implicit = true;
-        for (auto &gm : plan->gemms) all_implicit = all_implicit && gm.implicit;
-        if (ncls > 1 && ncls <= enn_b200_context::kAuxStreams + 1 && all_implicit && !ctx->opt("no_fan_out")) {
-            plan->fan_out = true;
-            const int share = ctx->launch_sms() / ncls > 0 ? ctx->launch_sms() / ncls : 1;
-            for (auto &gm : plan->gemms)
-                if (gm.grid > share) gm.grid = share;
-        }
     }
 
-    {   // All implicit GEMMs of an operator read the same input: one padded copy with the union of their margins.
-        int32_t lo_y = 0, lo_x = 0, hi_y = 0, hi_x = 0;
-        bool any = false;
-        for (auto &gm : plan->gemms)
-            if (gm.implicit && gm.padded) {
-                any = true;
-                lo_y = gm.pad_lo_y > lo_y ? gm.pad_lo_y : lo_y;
-                lo_x = gm.pad_lo_x > lo_x ? gm.pad_lo_x : lo_x;
-                const int32_t hy = gm.hp - gm.pad_lo_y - g.h, hx = gm.wp - gm.pad_lo_x - g.w;
-                hi_y = hy > hi_y ? hy : hi_y;
-                hi_x = hx > hi_x ? hx : hi_x;
-            }
-        if (any) {
-            bool first = true;
-            for (auto &gm : plan->gemms)
-                if (gm.implicit && gm.padded) {
-                    for (int32_t t = 0; t < gm.prm.taps; ++t) {
-                        gm.prm.tap_dy[t] = static_cast<int16_t>(gm.prm.tap_dy[t] + lo_y - gm.pad_lo_y);
-                        gm.prm.tap_dx[t] = static_cast<int16_t>(gm.prm.tap_dx[t] + lo_x - gm.pad_lo_x);
-                    }
-                    gm.pad_lo_y = lo_y; gm.pad_lo_x = lo_x;
-                    gm.hp = lo_y + g.h + hi_y; gm.wp = lo_x + g.w + hi_x;
-                    gm.runs_pad = first;
-                    first = false;
-                    const size_t need = static_cast<size_t>(g.n) * gm.hp * gm.wp * cin;
-                    if (need > plan->scratch_bytes) plan->scratch_bytes = need;
-                }
-        }
-    }
     if (plan->scratch_bytes > (static_cast<size_t>(8) << 30)) return bail(ENN_B200_INVALID_PARAMS);   // keep the direct kernel
     cudaError_t e;
     if ((plan->scratch_bytes && (e = cudaMalloc(&plan->scratch, plan->scratch_bytes)) != cudaSuccess) ||
@@ -2077,14 +1674,7 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
     int launches = 0;
     for (auto &gm : plan->gemms) {
         gm.prm.err = plan->err_dev;
-        launches += ((gm.gather && !gm.first_layer) || (gm.implicit && gm.runs_pad)) ? 2 : 1;
-        if (gm.implicit && gm.padded) {
-            if (!encode_nhwc(ctx, &gm.map_a, plan->scratch, cin, gm.wp, gm.hp, g.n, gm.prm.span, gm.prm.conv_wt, gm.prm.conv_ht)) {
-                ctx->last_error = "cuTensorMapEncodeTiled failed for the padded activation tensor";
-                return bail(ENN_B200_CUDA_FAILURE);
-            }
-            gm.map_a_ptr = plan->scratch;
-        }
+        launches += gm.gather && !gm.first_layer ? 2 : 1;
         if (gm.gather) {   // the offset table also serves as the fallback for misaligned input pointers
             // Byte-granular gather: per reduction index, the byte offset of (ky, kx, c) from the tap-(0,0) pixel
             // and the tap's pixel displacement.
@@ -2217,26 +1807,8 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
         return ENN_B200_CUDA_FAILURE;
     }
     if (plan->gc) return gconv_execute(op, plan, in, out);
-    #ifdef ENN_B200_DEV
-    const bool fan_out = plan->fan_out && !getenv("ENN_B200_TC_DEBUG");
-#else
-    const bool fan_out = plan->fan_out;
-#endif
-    if (fan_out && !ctx->aux_ready) {
-        bool ok = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) == cudaSuccess;
-        for (int i = 0; i < enn_b200_context::kAuxStreams && ok; ++i)
-            ok = cudaStreamCreateWithFlags(&ctx->aux_streams[i], cudaStreamNonBlocking) == cudaSuccess &&
-                 cudaEventCreateWithFlags(&ctx->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) {
-            ctx->last_error = "could not create the side streams";
-            return ENN_B200_CUDA_FAILURE;
-        }
-        ctx->aux_ready = true;
-    }
     const bool starve = plan->starve_next;
     plan->starve_next = false;
-    int cls = 0;             // index of the GEMM among those launched (fan-out: 0 runs on the main stream)
-    bool forked = false;
     for (auto &gm : plan->gemms) {
         TcParams &p = gm.prm;
         if (p.M == 0) continue;
@@ -2253,26 +1825,6 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
             const int64_t total16 = static_cast<int64_t>(p.M) * (gm.ig.Kp >> 4);
             const unsigned blocks = static_cast<unsigned>((total16 + 255) / 256);
             launch_im2col(gm.ig, in, static_cast<uint8_t *>(plan->scratch), total16, blocks, ctx->stream);
-        } else if (gm.implicit) {
-            if ((reinterpret_cast<uintptr_t>(in) & 15) != 0) {
-                ctx->last_error = "tensor-core path needs a 16-byte aligned input pointer";
-                return ENN_B200_INVALID_PARAMS;
-            }
-            const Im2colGeom &ig = gm.ig;
-            if (gm.padded && !gm.runs_pad) {
-                // the padded copy was written by an earlier GEMM of this operator in the same execute
-            } else if (gm.padded) {
-                const int64_t total16 = static_cast<int64_t>(ig.n) * gm.hp * gm.wp * (ig.cin >> 4);
-                pad_nhwc_kernel<<<static_cast<unsigned>((total16 + 255) / 256), 256, 0, ctx->stream>>>(
-                    static_cast<const uint8_t *>(in), static_cast<uint8_t *>(plan->scratch), ig.n, ig.h, ig.w, ig.cin, gm.hp, gm.wp, gm.pad_lo_y,
-                    gm.pad_lo_x, ig.fill, total16);
-            } else if (gm.map_a_ptr != in) {
-                if (!encode_nhwc(ctx, &gm.map_a, in, ig.cin, ig.w, ig.h, ig.n, p.span, p.conv_wt, p.conv_ht)) {
-                    ctx->last_error = "cuTensorMapEncodeTiled failed for the activation tensor";
-                    return ENN_B200_CUDA_FAILURE;
-                }
-                gm.map_a_ptr = in;
-            }
         } else {
             if ((reinterpret_cast<uintptr_t>(in) & 15) != 0) {
                 ctx->last_error = "tensor-core path needs a 16-byte aligned input pointer";
@@ -2325,23 +1877,7 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
             p.dbg = dbg_buf;
         }
 #endif
-        cudaStream_t gs = ctx->stream;
-        if (fan_out) {
-            if (!forked) {       // everything the classes read (input, padded copy) is ordered before this point
-                cudaEventRecord(ctx->ev_fork, ctx->stream);
-                forked = true;
-            }
-            if (cls > 0) {
-                gs = ctx->aux_streams[cls - 1];
-                cudaStreamWaitEvent(gs, ctx->ev_fork, 0);
-            }
-        }
-        launch_tc_gemm(gm, gm.map_a, p, gs);
-        if (fan_out && cls > 0) {
-            cudaEventRecord(ctx->ev_join[cls - 1], gs);
-            cudaStreamWaitEvent(ctx->stream, ctx->ev_join[cls - 1], 0);
-        }
-        ++cls;
+        launch_tc_gemm(gm, gm.map_a, p, ctx->stream);
 #ifdef ENN_B200_DEV
         if (dbg) {
             cudaStreamSynchronize(ctx->stream);

@@ -19,12 +19,6 @@ struct enn_b200_context {
     int cc_major = 0, cc_minor = 0;
     std::string last_error;
     void *encode_tiled = nullptr;   // cuTensorMapEncodeTiled, resolved through the runtime
-    // Side streams for operators made of independent launches (the parity classes of a transposed convolution): forked
-    // from and joined back into `stream` with events, created on first use.
-    static constexpr int kAuxStreams = 8;
-    cudaStream_t aux_streams[kAuxStreams] = {};
-    cudaEvent_t ev_fork = nullptr, ev_join[kAuxStreams] = {};
-    bool aux_ready = false;
     // Planner overrides set with enn_b200_context_set_option (tests and tuning).  They are read when an operator is
     // prepared, never on the execute path, and never from the environment.
     std::map<std::string, int> options;

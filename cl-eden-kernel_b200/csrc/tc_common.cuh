@@ -94,12 +94,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
                  : "memory");
 }
 
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
-
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -189,22 +183,6 @@ __device__ __forceinline__ void umma_i8_run(uint32_t d_tmem, uint32_t desc_hi, u
 #undef ENN_MMA_PAIR
 }
 
-__device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_x1(uint32_t taddr, uint32_t &r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major operand tile in shared memory, 128-byte rows, 128B swizzle: rows are 128 bytes apart, groups of 8
@@ -306,9 +284,9 @@ __device__ __forceinline__ int32_t tc_requant(int32_t acc, const int4 &c, int32_
     return tc_requant<MODE>(acc, cr, hi_clamp, out_zp, act_min, act_max);
 }
 
-// Fused add: the 16 requantised bytes of a chunk (four words) and the 16 bytes of the other addend at the same place go
-// through the quantized add exactly as add_kernel_vec computes it (kernels_direct.cu): stage 1 of either input from the
-// operator's tables in shared memory, stage 2 computed.
+// Fused add: four requantised bytes and the four bytes of the other addend at the same place go through the quantized add
+// exactly as add_kernel_vec computes it (kernels_direct.cu): stage 1 of either input from the operator's tables in shared
+// memory, stage 2 computed.
 struct FaddCtx {
     uint32_t lut_u32;       // 2 x 256 words in shared memory: input-0 table, input-1 table
     int32_t mo, so, out_off, act_min, act_max;
@@ -330,12 +308,170 @@ __device__ __forceinline__ uint32_t fadd_word(uint32_t y, uint32_t r, const Fadd
     }
     return word;
 }
-__device__ __forceinline__ void fadd_chunk(uint32_t (&w)[4], const uint8_t *res, const FaddCtx &f) {
-    const uint4 r = *reinterpret_cast<const uint4 *>(res);      // plain load: the output may be written over this addend
-    w[0] = fadd_word(w[0], r.x, f);
-    w[1] = fadd_word(w[1], r.y, f);
-    w[2] = fadd_word(w[2], r.z, f);
-    w[3] = fadd_word(w[3], r.w, f);
+// ---------------------------------------------------------------------------------------------------------------------
+// Epilogue of one accumulator tile, "quad" form.
+//
+// tcgen05.ld 16x256b hands a thread the two columns 2q, 2q + 1 (q = lane & 3) of every group of eight for the rows
+// lane / 4 and lane / 4 + 8, so a warp's quarter of the tile (32 rows) gives a thread FOUR rows of the same columns.  The
+// constants of a column are then loaded from shared memory once per four outputs instead of once per output: with one row
+// per thread (32x32b) those 16-byte loads, two to four data cycles of the load-store unit each, were what bounded every
+// epilogue (75 % of that unit's cycles in the 3x3 layer 256x56x56x64).  The planners permute the channels within groups of 32
+// so that a thread's eight columns of a group are eight consecutive output channels: a quad stores whole 32-byte sectors.
+//
+// Channel c of an N tile of bn_data channels (bn_data % 16 == 0; a last group of 16 uses four channels per thread):
+//   tile_row   row of the packed weights = accumulator column
+//   tile_slot  position of its constants: the four threads of a quad read 64 consecutive bytes
+// ---------------------------------------------------------------------------------------------------------------------
+__host__ __device__ __forceinline__ int tile_row(int c, int bn_data) {
+    const int g = c & ~31, r = c & 31;
+    if (g + 32 <= bn_data) return g + 8 * ((r & 7) >> 1) + 2 * (r >> 3) + (r & 1);
+    return g + 8 * ((r & 3) >> 1) + 2 * ((r >> 2) & 3) + (r & 1);
+}
+__host__ __device__ __forceinline__ int tile_slot(int c, int bn_data) {
+    const int g = c & ~31, r = c & 31;
+    return g + 32 <= bn_data ? g + 4 * (r & 7) + (r >> 3) : g + 4 * (r & 3) + ((r >> 2) & 3);
+}
+
+__device__ __forceinline__ void tmem_ld_16x256_x1(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+// 8 * NJ columns of 16 rows, NJ = 2 or 4: r[4 * j + 2 * h + s] = row lane / 4 + 8 * h, column 8 * j + 2 * (lane & 3) + s.
+template <int NJ>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[4 * NJ]) {
+    if constexpr (NJ == 4)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                       "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr)
+                     : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+}
+
+// What the epilogue of a kernel needs to know once.
+struct EpiArgs {
+    int32_t hi_clamp, out_zp, act_min, act_max;
+    uint32_t lo_word, sign_word;    // lower clamp added back to the packed bytes, sign flip of signed outputs
+    int align;                      // widest store every row start allows: 8, 4 or 1
+    ptrdiff_t res_delta;            // fused add: the other addend relative to the output
+    FaddCtx fadd;
+};
+// ... and once per tile.
+struct EpiTile {
+    uint8_t *row[4];        // first output byte of this thread's rows (tile column 0), rows lane / 4 + 8 * h of the quarter
+    uint32_t live;          // bit h: row h exists
+    int32_t asum[4];        // zw' * sum_k a of the rows
+    int n_left;             // real columns of the tile
+};
+
+// P: the kernel's parameters.  Unsigned outputs: byte + act_min <= act_max <= 255, so a plain 32-bit add of the lower clamp never
+// carries between bytes.  Signed outputs (act_min may be negative): the bytes get act_min + 128 (0..127, sums again <= 255)
+// and the sign bit of every byte is flipped afterwards.
+template <typename P>
+__device__ __forceinline__ EpiArgs epi_args(const P &p, int64_t st_bits, ptrdiff_t res_delta, const FaddCtx &fadd) {
+    EpiArgs e;
+    e.hi_clamp = p.act_max - p.act_min;
+    e.out_zp = p.out_zp; e.act_min = p.act_min; e.act_max = p.act_max;
+    e.sign_word = p.a_signed ? 0x80808080u : 0u;
+    e.lo_word = (static_cast<uint32_t>(p.act_min + (p.a_signed ? 128 : 0)) & 0xff) * 0x01010101u;
+    e.align = (st_bits & 7) == 0 ? 8 : ((st_bits & 3) == 0 ? 4 : 1);
+    e.res_delta = res_delta;
+    e.fadd = fadd;
+    return e;
+}
+
+// Requantises columns [c0, c0 + 8 * NJ) of the warp's 32 rows and stores them.  `t_row`: TMEM address of the tile's column
+// 0 in the warp's lane quarter; `cols`: the tile's constants in shared memory.  FULL: every row and column is real and rows
+// start on 8-byte boundaries; the general form's tests (per row and store width) cost as much as the requantisation itself.
+template <int MODE, bool ASUM, bool FADD, int NJ, bool FULL>
+__device__ __forceinline__ void epi_group(uint32_t t_row, const uint8_t *cols, int c0, const EpiTile &t, int lane, const EpiArgs &e) {
+    constexpr bool kPlainPack = MODE == kModeReluSat;      // packed bytes are final: no lower clamp to add, no sign flip
+    constexpr int kCh = 2 * NJ;                            // consecutive channels per thread: 8 or 4
+    const int q = lane & 3;
+    uint32_t r[2][4 * NJ];
+    tmem_ld_16x256<NJ>(t_row + c0, r[0]);
+    tmem_ld_16x256<NJ>(t_row + (16u << 16) + c0, r[1]);
+    tmem_ld_wait();
+    const uint8_t *cp = cols + (c0 + q) * 16;
+    uint32_t w[4][kCh / 4];
+#pragma unroll
+    for (int i4 = 0; i4 < kCh / 4; ++i4) {
+        int32_t y[4][4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int i = 4 * i4 + b;
+            ColRegs cv;
+            ld_col_shared<MODE>(cp + i * 64, cv);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                int32_t acc = static_cast<int32_t>(r[h >> 1][4 * (i >> 1) + 2 * (h & 1) + (i & 1)]);
+                if (ASUM) acc -= t.asum[h];
+                y[h][b] = tc_requant<MODE>(acc, cv, e.hi_clamp, e.out_zp, e.act_min, e.act_max);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t hi = pack_sat_u8_tc(y[h][3], y[h][2], 0);
+            const uint32_t pk = pack_sat_u8_tc(y[h][1], y[h][0], hi);
+            w[h][i4] = kPlainPack ? pk : ((pk + e.lo_word) ^ e.sign_word);
+        }
+    }
+    const int cb = c0 + kCh * q;                            // this thread's first column
+    const int left = FULL ? kCh : t.n_left - cb;            // how many real ones from there on
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        if (!FULL && !(t.live >> h & 1)) continue;
+        uint8_t *o = t.row[h] + cb;
+        if constexpr (FADD) {                               // rows of 16-byte multiples only (plan)
+            if (left >= kCh) {
+                const uint8_t *res = o + e.res_delta;
+#pragma unroll
+                for (int k = 0; k < kCh / 4; ++k) w[h][k] = fadd_word(w[h][k], *reinterpret_cast<const uint32_t *>(res + 4 * k), e.fadd);
+            }
+        }
+        if (FULL || (left >= kCh && e.align >= kCh)) {
+            if constexpr (NJ == 4) *reinterpret_cast<uint2 *>(o) = make_uint2(w[h][0], w[h][1]);
+            else *reinterpret_cast<uint32_t *>(o) = w[h][0];
+        } else if (e.align >= 4 && (left & 3) == 0) {
+#pragma unroll
+            for (int k = 0; k < kCh / 4; ++k)
+                if (4 * k < left) *reinterpret_cast<uint32_t *>(o + 4 * k) = w[h][k];
+        } else {
+#pragma unroll
+            for (int b = 0; b < kCh; ++b)
+                if (b < left) o[b] = static_cast<uint8_t>(w[h][b >> 2] >> (8 * (b & 3)));
+        }
+    }
+}
+
+// Column groups first, first + step, ... of a tile of bn_data columns for the warp's 32 rows.  cols_of(c0) returns the
+// pointer the constants of columns c0 ... lie behind (at entry c0).
+template <int MODE, bool ASUM, bool FADD, typename ColsOf>
+__device__ __forceinline__ void epi_tile(uint32_t t_row, int first, int step, int bn_data, const EpiTile &t, int lane, const EpiArgs &e, ColsOf cols_of) {
+    const bool rows_full = __all_sync(0xffffffffu, t.live == 15u) && e.align == 8;
+    int c0 = first * 32;
+    if (rows_full)
+        for (; c0 + 32 <= t.n_left; c0 += 32 * step) epi_group<MODE, ASUM, FADD, 4, true>(t_row, cols_of(c0), c0, t, lane, e);
+    for (; c0 < t.n_left; c0 += 32 * step) {
+        if (c0 + 32 <= bn_data) epi_group<MODE, ASUM, FADD, 4, false>(t_row, cols_of(c0), c0, t, lane, e);
+        else epi_group<MODE, ASUM, FADD, 2, false>(t_row, cols_of(c0), c0, t, lane, e);
+    }
+}
+
+// zw' * sum_k a of this thread's four rows: accumulator column `col` of the extra group of 16.
+__device__ __forceinline__ void epi_asum(uint32_t t_row, int col, int32_t zw_eff, int lane, int32_t (&asum)[4]) {
+    uint32_t a[4], b[4];
+    tmem_ld_16x256_x1(t_row + col, a);
+    tmem_ld_16x256_x1(t_row + (16u << 16) + col, b);
+    tmem_ld_wait();
+    const int src = lane & ~3;      // column 0 of the group sits in the quad's first thread
+    asum[0] = zw_eff * static_cast<int32_t>(__shfl_sync(0xffffffffu, a[0], src));
+    asum[1] = zw_eff * static_cast<int32_t>(__shfl_sync(0xffffffffu, a[2], src));
+    asum[2] = zw_eff * static_cast<int32_t>(__shfl_sync(0xffffffffu, b[0], src));
+    asum[3] = zw_eff * static_cast<int32_t>(__shfl_sync(0xffffffffu, b[2], src));
 }
 
 }  // namespace
