@@ -467,6 +467,34 @@ static int32_t conv_like_prepare_const(enn_b200_context *ctx, const enn_b200_con
             dw_ring_plan(op);
         }
     }
+    if (kind == OP_DEPTHWISE && !op->dw_chan && dw_quad_eligible(g)) {
+        // Constants of the channel-quad kernel (depthwise.cu): signed weight bytes, four taps of a channel per word.
+        std::vector<int32_t> mult, shift;
+        derive_requant(cout, d->per_channel != 0, d->in_scale, d->w_scale, d->bias_scale, d->out_scale, pc_scales, &mult, &shift);
+        const int32_t taps = g.kh * g.kw, zw = g.w_signed ? g.w_zp : g.w_zp - 128;
+        std::vector<uint32_t> wp(static_cast<size_t>((taps + 3) / 4) * cout, 0);
+        std::vector<int32_t> chan(static_cast<size_t>(cout) * 4, 0);
+        for (int32_t c = 0; c < cout; ++c) {
+            int64_t wsum = 0;
+            for (int32_t t = 0; t < taps; ++t) {
+                const uint8_t raw = packed[static_cast<size_t>(t) * cout + c], wv = g.w_signed ? raw : raw ^ 0x80;
+                wsum += static_cast<int8_t>(wv);
+                wp[static_cast<size_t>(t >> 2) * cout + c] |= static_cast<uint32_t>(wv) << (8 * (t & 3));
+            }
+            const int64_t folded = static_cast<int64_t>(bias_host[c]) - static_cast<int64_t>(g.in_zp) * wsum + static_cast<int64_t>(taps) * g.in_zp * zw;
+            chan[c * 4] = mult[c];
+            chan[c * 4 + 1] = shift[c];
+            chan[c * 4 + 2] = static_cast<int32_t>(static_cast<uint32_t>(static_cast<uint64_t>(folded)));     // sums are modulo 2^32
+        }
+        int32_t *dc = nullptr;
+        uint32_t *dwp = nullptr;
+        if ((st = upload_vec(op, chan, &dc)) || (st = upload_vec(op, wp, &dwp))) {
+            enn_b200_op_release(op);
+            return st;
+        }
+        op->dwq_chan = dc;
+        op->dwq_w = dwp;
+    }
     if (kind != OP_DEPTHWISE && tc_available(ctx)) {
         st = tc_plan_conv(op, packed.data());
         if (st == ENN_B200_SUCCESS && op->tc) op->impl = ENN_B200_IMPL_TCGEN05;
@@ -703,6 +731,10 @@ int32_t enn_b200_op_execute(enn_b200_op *op, const void *in, void *out) {
             if (op->dw_chan && op->impl == ENN_B200_IMPL_DEPTHWISE &&
                 ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 3) == 0) {
                 e = launch_dw3x3(op->g, op->dw_chan, op->dw_relu, op->dw_w, in, out, ctx->sm_count, ctx->stream);
+                break;
+            }
+            if (op->dwq_w && op->impl == ENN_B200_IMPL_DEPTHWISE && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 3) == 0) {
+                e = launch_dw_quad(op->g, op->dwq_chan, op->dwq_w, in, out, ctx->stream);
                 break;
             }
             e = launch_depthwise(op->g, op->rq, in, op->w_direct, out, ctx->sm_count, ctx->stream);

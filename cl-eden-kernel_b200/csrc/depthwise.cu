@@ -1,11 +1,12 @@
 // DepthwiseConv2D, NHWC.  Value: DepthwiseconvolutionKernels.cpp:1273-1371 after the zero-point `pad`
 // pre-pass (border taps contribute nothing).  HBM-bound: no tensor cores.
 //
-// Two kernels:
+// Kernels:
 //   depthwise_generic_kernel  any kernel size / stride / dilation / depth multiplier / signedness;
 //   dw3x3_kernel              3x3, stride 1 or 2, dilation 1, multiplier 1, C % 4 == 0, u8 activations: the
 //                             case every reference 3x3 variant (depthwise_conv_3x3s1_pad_merge, ..3x3s2..,
 //                             depthwise_conv_per_channel) covers and the one the benchmark configuration uses.
+// Between them: depthwise_quad_kernel, any kernel size / stride / dilation / signedness with multiplier 1 and C % 4 == 0.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -838,6 +839,132 @@ cudaError_t launch_dw3x3(const ConvGeom &g, const void *chan, bool relu_form, co
     }
 #undef ENN_DW_LAUNCH
     return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------------------------------------
+// Four channels at a time, any taps: what the 3x3 kernels do not take (5x5, dilation, signed activations, left shifts), for
+// multiplier 1 and C % 4 == 0.
+//
+// The general kernel spends about thirty instructions per tap and output on byte loads and 64-bit addresses.  Here a thread owns
+// a channel quad of kDwQuadPixels neighbouring output pixels; the words of four taps (border positions: the input zero point) are
+// byte-transposed so that one dp4a covers four taps of a channel: 4 loads, 8 PRMT and 4 dp4a for 16 multiply-adds, and the packed
+// weights of a tap group are one 16-byte load shared by the pixels.  Weights are signed bytes w' (u8: w - 128, zero point
+// zw' = zw - 128); sum (a - za)(w - zw) = sum a w' - zw' sum a + (K za zw' - za sum w'), the bracket folded into the bias.
+// Modulo 2^32 all of this equals the general kernel's sum, and the requantisation is the same function.
+// Bound by integer issue (about eight instructions per tap and quad).  16 x 56 x 56 x 96, general kernel -> this one: 5x5 u8
+// 234 -> 28.1 us, 3x3 int8 activations 123 -> 15.7 us; 1 x 14 x 14 x 240 5x5 10.3 -> 4.6 us.
+// ------------------------------------------------------------------------------------------------------
+constexpr int kDwQuadPixels = 2;
+
+template <bool A_SIGNED>
+__device__ __forceinline__ int32_t dp4a_as8(uint32_t a, uint32_t w, int32_t c) {
+    int32_t d;
+    if (A_SIGNED) asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(w), "r"(c));
+    else asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(w), "r"(c));
+    return d;
+}
+
+// KS: kernel size 3 or 5 (taps unrolled), 0: any.  taps4: [ceil(K / 4)][C] words, chan: [C] {multiplier, shift, folded bias, -}.
+template <int KS, bool A_SIGNED, bool NEED_ASUM>
+__global__ void __launch_bounds__(256)
+depthwise_quad_kernel(ConvGeom g, const int4 *__restrict__ chan, const uint32_t *__restrict__ taps4, int32_t zw,
+                      const uint8_t *__restrict__ in, uint8_t *__restrict__ out, uint32_t total) {
+    pdl_trigger();
+    const uint32_t idx = blockIdx.x * 256u + threadIdx.x;
+    if (idx >= total) return;
+    const uint32_t cqn = static_cast<uint32_t>(g.cin) >> 2, oxn = (static_cast<uint32_t>(g.ow) + kDwQuadPixels - 1) / kDwQuadPixels;
+    const uint32_t cq = idx % cqn, t0 = idx / cqn, oxg = t0 % oxn, t1 = t0 / oxn;
+    const int oy = static_cast<int>(t1 % static_cast<uint32_t>(g.oh)), b = static_cast<int>(t1 / static_cast<uint32_t>(g.oh));
+    const int ox0 = static_cast<int>(oxg) * kDwQuadPixels;
+    const int kh = KS ? KS : g.kh, kw = KS ? KS : g.kw, taps = kh * kw;
+    const uint32_t zaw = (static_cast<uint32_t>(g.in_zp) & 0xff) * 0x01010101u;
+    const int iy0 = oy * g.sh - g.pt, ix0 = ox0 * g.sw - g.pl;
+    const uint8_t *img = in + static_cast<int64_t>(b) * g.h * g.w * g.cin + cq * 4;
+    int32_t acc[kDwQuadPixels][4] = {}, asum[kDwQuadPixels][4] = {};
+    pdl_wait();
+    int ky = 0, kx = 0;
+    auto group = [&](int t) {       // taps t .. t + 3
+        const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(taps4 + static_cast<size_t>(t >> 2) * g.cin) + cq);
+        uint32_t a[kDwQuadPixels][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int iy = iy0 + ky * g.dh;
+            const bool row_ok = t + i < taps && static_cast<uint32_t>(iy) < static_cast<uint32_t>(g.h);
+#pragma unroll
+            for (int p = 0; p < kDwQuadPixels; ++p) {
+                const int ix = ix0 + p * g.sw + kx * g.dw;
+                a[p][i] = t + i < taps ? zaw : 0u;
+                if (row_ok && static_cast<uint32_t>(ix) < static_cast<uint32_t>(g.w))
+                    a[p][i] = __ldg(reinterpret_cast<const uint32_t *>(img + (static_cast<int64_t>(iy) * g.w + ix) * g.cin));
+            }
+            if (++kx == kw) {
+                kx = 0;
+                ++ky;
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < kDwQuadPixels; ++p) {
+            const uint32_t u0 = prmt(a[p][0], a[p][1], 0x5140), u1 = prmt(a[p][0], a[p][1], 0x7362);
+            const uint32_t u2 = prmt(a[p][2], a[p][3], 0x5140), u3 = prmt(a[p][2], a[p][3], 0x7362);
+            const uint32_t c0 = prmt(u0, u2, 0x5410), c1 = prmt(u0, u2, 0x7632), c2 = prmt(u1, u3, 0x5410), c3 = prmt(u1, u3, 0x7632);
+            acc[p][0] = dp4a_as8<A_SIGNED>(c0, wv.x, acc[p][0]);
+            acc[p][1] = dp4a_as8<A_SIGNED>(c1, wv.y, acc[p][1]);
+            acc[p][2] = dp4a_as8<A_SIGNED>(c2, wv.z, acc[p][2]);
+            acc[p][3] = dp4a_as8<A_SIGNED>(c3, wv.w, acc[p][3]);
+            if (NEED_ASUM) {
+                asum[p][0] = dp4a_as8<A_SIGNED>(c0, 0x01010101u, asum[p][0]);
+                asum[p][1] = dp4a_as8<A_SIGNED>(c1, 0x01010101u, asum[p][1]);
+                asum[p][2] = dp4a_as8<A_SIGNED>(c2, 0x01010101u, asum[p][2]);
+                asum[p][3] = dp4a_as8<A_SIGNED>(c3, 0x01010101u, asum[p][3]);
+            }
+        }
+    };
+    if constexpr (KS != 0) {
+#pragma unroll
+        for (int t = 0; t < KS * KS; t += 4) group(t);
+    } else {
+        for (int t = 0; t < taps; t += 4) group(t);
+    }
+    uint8_t *o = out + ((static_cast<int64_t>(b) * g.oh + oy) * g.ow + ox0) * g.cin + cq * 4;
+    uint32_t word[kDwQuadPixels] = {};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int4 k = __ldg(chan + cq * 4 + c);
+#pragma unroll
+        for (int p = 0; p < kDwQuadPixels; ++p) {
+            uint32_t s = static_cast<uint32_t>(acc[p][c]) + static_cast<uint32_t>(k.z);
+            if (NEED_ASUM) s -= static_cast<uint32_t>(zw) * static_cast<uint32_t>(asum[p][c]);
+            word[p] |= (static_cast<uint32_t>(enn_requant(static_cast<int32_t>(s), k.x, k.y, g.out_zp, g.act_min, g.act_max)) & 0xff) << (8 * c);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < kDwQuadPixels; ++p)
+        if (ox0 + p < g.ow) *reinterpret_cast<uint32_t *>(o + static_cast<int64_t>(p) * g.cin) = word[p];
+}
+
+// Multiplier 1, channel quads, and a thread count that fits 31 bits.
+bool dw_quad_eligible(const ConvGeom &g) {
+    return g.groups == 1 && g.cout == g.cin && (g.cin & 3) == 0 && static_cast<int64_t>(g.n) * g.oh * g.ow * (g.cin >> 2) < (1ll << 31) - 256;
+}
+
+cudaError_t launch_dw_quad(const ConvGeom &g, const void *chan, const void *taps4, const void *in, void *out, cudaStream_t s) {
+    const int64_t total = static_cast<int64_t>(g.n) * g.oh * ((g.ow + kDwQuadPixels - 1) / kDwQuadPixels) * (g.cin >> 2);
+    if (total == 0) return cudaSuccess;
+    const int32_t zw = g.w_signed ? g.w_zp : g.w_zp - 128;
+    const dim3 blocks(static_cast<unsigned>((total + 255) / 256));
+    const int4 *c = static_cast<const int4 *>(chan);
+    const uint32_t *w = static_cast<const uint32_t *>(taps4);
+    const uint8_t *i = static_cast<const uint8_t *>(in);
+    uint8_t *o = static_cast<uint8_t *>(out);
+    const uint32_t n = static_cast<uint32_t>(total);
+#define ENN_DWQ(KS)                                                                                                    \
+    (g.a_signed ? (zw ? launch_pdl(depthwise_quad_kernel<KS, true, true>, blocks, dim3(256), 0, s, g, c, w, zw, i, o, n)    \
+                      : launch_pdl(depthwise_quad_kernel<KS, true, false>, blocks, dim3(256), 0, s, g, c, w, zw, i, o, n))  \
+                : (zw ? launch_pdl(depthwise_quad_kernel<KS, false, true>, blocks, dim3(256), 0, s, g, c, w, zw, i, o, n)   \
+                      : launch_pdl(depthwise_quad_kernel<KS, false, false>, blocks, dim3(256), 0, s, g, c, w, zw, i, o, n)))
+    const int ks = g.kh == g.kw ? g.kh : 0;
+    return ks == 3 ? ENN_DWQ(3) : (ks == 5 ? ENN_DWQ(5) : ENN_DWQ(0));
+#undef ENN_DWQ
 }
 
 cudaError_t launch_depthwise(const ConvGeom &g, const Requant &rq, const void *in, const void *w, void *out,

@@ -111,6 +111,7 @@ struct enn_b200_op {
     void *dw_chan = nullptr;           // depthwise 3x3 fast path: per-channel constants (in `owned`)
     bool dw_relu = false;              // dw_chan holds the merged ReLU form {C low, C high, M0, e - 1}
     void *dw_w = nullptr;              // depthwise 3x3 fast path: packed 3-tap weight words (in `owned`)
+    void *dwq_chan = nullptr, *dwq_w = nullptr;   // depthwise channel-quad kernel: constants and packed taps (in `owned`)
     void *dw_ring = nullptr;           // depthwise row-ring plan (depthwise.cu), owned
     void *tc = nullptr;                // tensor-core plan (gemm_tc.cu), owned
     void *graph_state = nullptr;       // state of Mean / Concat / Softmax / Resize (graph_ops.cu), owned
@@ -132,6 +133,8 @@ cudaError_t launch_depthwise(const ConvGeom &g, const Requant &rq, const void *i
 bool dw3x3_eligible(const ConvGeom &g);
 cudaError_t launch_dw3x3(const ConvGeom &g, const void *chan, bool relu_form, const void *w_packed, const void *in, void *out,
                          int sm_count, cudaStream_t s);
+bool dw_quad_eligible(const ConvGeom &g);
+cudaError_t launch_dw_quad(const ConvGeom &g, const void *chan, const void *taps4, const void *in, void *out, cudaStream_t s);
 bool dw_ring_plan(enn_b200_op *op);
 cudaError_t dw_ring_launch(enn_b200_op *op, const void *in, void *out);
 void dw_ring_release(enn_b200_op *op);

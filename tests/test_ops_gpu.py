@@ -236,6 +236,31 @@ def test_depthwise_parity(enn, orc, ctx, name):
         op.release()
 
 
+# Channel-quad kernel: unrolled 3x3 and 5x5 and other sizes (tap groups with 1, 2 and 3 taps left over), strides, dilation, signed
+# activations, both weight kinds, a last pixel without a partner, images smaller than the filter.
+DW_QUAD_CASES = {
+    "k5_u8": dict(n=2, h=13, w=17, c=24, k=5, out_scale=0.2),
+    "k5_s2_pt_s8": dict(n=3, h=15, w=14, c=20, k=5, stride=2, per_channel=False, act_dtype=cases.enn.S8, in_zp=-9, out_zp=-128, out_scale=0.1),
+    "k3_s8": dict(n=2, h=19, w=21, c=40, act_dtype=cases.enn.S8, in_zp=3, out_zp=-5, act=cases.enn.ACT_NONE, out_scale=0.3),
+    "k3_s2_s8_pt": dict(n=1, h=9, w=31, c=4, stride=2, per_channel=False, act_dtype=cases.enn.S8, in_zp=-128, out_zp=-128),
+    "k3_dil2": dict(n=2, h=11, w=10, c=16, dil=2, out_scale=0.1),
+    "k7_small_image": dict(n=2, h=3, w=5, c=12, k=7, per_channel=False, in_zp=0, out_scale=0.2),
+    "k2": dict(n=2, h=8, w=9, c=32, k=2, stride=2),
+    "k1": dict(n=1, h=6, w=7, c=8, k=1, in_zp=255),
+    "k3_left_shift": dict(n=1, h=9, w=9, c=16, out_scale=2e-5, act=cases.enn.ACT_NONE, out_zp=100),
+}
+
+
+@pytest.mark.parametrize("name", list(DW_QUAD_CASES))
+def test_depthwise_channel_quads(enn, orc, ctx, name):
+    d, x, w, b, sc = cases.depthwise_case(seed=_seed("dwq_" + name), **DW_QUAD_CASES[name])
+    op = enn.depthwise(ctx, d, w, b, sc)
+    try:
+        _check(op, orc.depthwise(d, x, w, b, sc), x)
+    finally:
+        op.release()
+
+
 @pytest.mark.parametrize("seed", range(16))
 def test_depthwise_parity_sweep(enn, orc, ctx, seed):
     """Pseudo-random 3x3 depthwise layers (channels, stride, activation, zero points, output scale over three decades,
