@@ -445,15 +445,6 @@ dw3x3_ring_kernel(const DwRingParams p, const DwChan *__restrict__ chan, const u
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {   // every slot starts as zero points; the copies overwrite the in-image pixel range only
-        const uint32_t zaw = (static_cast<uint32_t>(p.in_zp) & 0xff) * 0x01010101u;
-        const uint32_t n16 = static_cast<uint32_t>(p.nr) * (p.pitch >> 4);
-        for (uint32_t i = tid; i < n16; i += blockDim.x)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ring + i * 16), "r"(zaw) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // ordered before the bulk copies into the same bytes
-    }
-    __syncthreads();
-
     // This CTA: x tile `tx`, output rows [u0, u1) of the N * OH rows of that tile column (row u = image * OH + oy).
     const int tx = static_cast<int>(blockIdx.x) / p.ctas_per_tx, part = static_cast<int>(blockIdx.x) - tx * p.ctas_per_tx;
     const int64_t units = static_cast<int64_t>(p.n) * p.oh;
@@ -462,6 +453,15 @@ dw3x3_ring_kernel(const DwRingParams p, const DwChan *__restrict__ chan, const u
     const int ix_start = ox0 * STRIDE - p.pl;
     const int ix_lo = ix_start < 0 ? 0 : ix_start;
     const int ix_hi = ix_start + p.slot_px < p.w ? ix_start + p.slot_px : p.w;
+    {   // pixels left and right of the image, which no copy ever writes, hold the zero point in every slot; most tiles have none
+        const uint32_t zaw = (static_cast<uint32_t>(p.in_zp) & 0xff) * 0x01010101u, c16 = static_cast<uint32_t>(p.c) >> 4;
+        const uint32_t left = static_cast<uint32_t>(ix_lo - ix_start) * c16, end = static_cast<uint32_t>(ix_hi - ix_start) * c16;
+        const uint32_t border = left + static_cast<uint32_t>(p.slot_px) * c16 - end;
+        for (uint32_t s = static_cast<uint32_t>(warp); s < static_cast<uint32_t>(p.nr); s += blockDim.x >> 5)
+            for (uint32_t i = static_cast<uint32_t>(lane); i < border; i += 32)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ring + s * p.pitch + (i < left ? i : i - left + end) * 16), "r"(zaw) : "memory");
+    }
+    __syncthreads();
 
     if (warp == ncw) {
         // ---------------- producer: one bulk copy per input row, in the order the consumers take them ----------------
@@ -696,6 +696,8 @@ bool dw_ring_plan(enn_b200_op *op) {
     if (ns_max > strips) ns_max = strips;
     const int tx_n = (strips + ns_max - 1) / ns_max;
     const int ns = (strips + tx_n - 1) / tx_n;
+    // every x tile must hold at least one pixel of the image: a tile without one has no copies and nothing to wait for
+    if ((tx_n - 1) * ns * 4 * s - g.pl >= g.w || (4 * ns - 1) * s + 3 <= g.pl) return false;
     DwRingPlan *pl = new (std::nothrow) DwRingPlan();
     if (!pl) return false;
     DwRingParams &p = pl->prm;
@@ -721,11 +723,14 @@ bool dw_ring_plan(enn_b200_op *op) {
     }
     p.nr = nr;
     p.in_zp = g.in_zp; p.w_zp = g.w_zp; p.act_min = g.act_min; p.act_max = g.act_max;
-    // One wave of CTAs, each with at least a few output rows so that the two halo rows stay cheap.
+    // One wave of CTAs, each with at least six output rows so that the two halo rows stay cheap; fewer where six would leave
+    // SMs without a CTA (a CTA's rows come one after another, the halo rows come out of the L2): MobileNetV2 at one image
+    // 325.5 -> 299.4 us, the lists' other kernels unchanged.
     const int64_t units = static_cast<int64_t>(g.n) * g.oh;
     int per_tx = (per_sm * ctx->launch_sms()) / tx_n;
     if (per_tx < 1) per_tx = 1;
-    const int64_t min_rows = 6;
+    const int64_t per_sm_rows = units * tx_n / ctx->launch_sms();
+    const int64_t min_rows = per_sm_rows >= 6 ? 6 : (per_sm_rows < 1 ? 1 : per_sm_rows);
     if (per_tx > (units + min_rows - 1) / min_rows) per_tx = static_cast<int>((units + min_rows - 1) / min_rows);
     p.ctas_per_tx = per_tx;
     pl->grid = per_tx * tx_n;

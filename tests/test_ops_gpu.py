@@ -261,6 +261,28 @@ def test_depthwise_channel_quads(enn, orc, ctx, name):
         op.release()
 
 
+@pytest.mark.parametrize("kw", [dict(n=1, h=7, w=7, c=960), dict(n=1, h=112, w=112, c=32), dict(n=2, h=30, w=29, c=144, stride=2), dict(n=1, h=61, w=300, c=16)])
+def test_depthwise_ring_few_rows_per_cta(enn, orc, ctx, kw):
+    """Launches with fewer than six output rows per CTA, and x tiles with and without border pixels."""
+    d, x, w, b, sc = cases.depthwise_case(seed=77, **kw)
+    op = enn.depthwise(ctx, d, w, b, sc)
+    try:
+        _check(op, orc.depthwise(d, x, w, b, sc), x)
+    finally:
+        op.release()
+
+
+def test_depthwise_tiles_in_the_padding(enn, orc, ctx):
+    """Padding wider than an x tile: the row ring would have tiles without a single pixel of the image."""
+    d, x, w, b, sc = cases.depthwise_case(seed=78, n=1, h=9, w=20, c=32)
+    d.pad_r = 150
+    op = enn.depthwise(ctx, d, w, b, sc)
+    try:
+        _check(op, orc.depthwise(d, x, w, b, sc), x)
+    finally:
+        op.release()
+
+
 @pytest.mark.parametrize("seed", range(16))
 def test_depthwise_parity_sweep(enn, orc, ctx, seed):
     """Pseudo-random 3x3 depthwise layers (channels, stride, activation, zero points, output scale over three decades,
