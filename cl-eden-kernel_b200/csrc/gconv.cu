@@ -102,7 +102,7 @@ struct UnitWalk {
 //   G < 16   8- or 4-byte loads into registers, all of a k-block in flight, then stores, fence, one arrival per warp.
 //            Asynchronous copies of 8 bytes took 27 SM cycles per warp instruction (16 bytes: 10), loads and stores 4 to 6.
 template <int G>
-__device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, uint32_t base, uint32_t full0, uint32_t empty0,
+__device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, const uint8_t *sp, uint32_t base, uint32_t full0, uint32_t empty0,
                                             volatile int *abort_flag, bool starve) {
     constexpr int kPerRow = kBK / G;                            // copies per A row and k-block: 8, 16 or 32
     constexpr int kRowsPerPass = kGatherThreads / kPerRow;      // 16, 8 or 4
@@ -122,6 +122,7 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
     constexpr int kRowsPerWarp = 32 / kPerRow;                  // 4, 2 or 1
     const int wbase = (t >> 5) * kRowsPerWarp;
     const uint32_t rt = base + L.rows + static_cast<uint32_t>(t >> 5) * 512u, rt_lane = rt + static_cast<uint32_t>(lane / kPerRow) * 16;
+    const int2 *const tab0 = (p.tab_entries ? reinterpret_cast<const int2 *>(sp + L.tab) : p.tab) + piece;
     uint32_t stage = 0, phase = 0;
     bool ok = !starve;
     UnitWalk u;
@@ -150,12 +151,21 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(roff[i]), "=r"(riy[i]), "=r"(rix[i]), "=r"(pad) : "r"(rt_lane + i * kRowsPerWarp * 16));
             }
         }
+        const int2 *tab = tab0 + c.tab0;
         for (int kb = 0; kb < c.k_blocks; ++kb) {
             if (lane == 0) ok = mbar_test_wait(empty0 + 8 * stage, phase ^ 1) || mbar_wait_fast(empty0 + 8 * stage, phase ^ 1, abort_flag, p.err, 1);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
-            int toff, tyx;
-            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(toff), "=r"(tyx) : "r"(base + L.tab + (c.tab0 + kb * kPerRow + piece) * 8));
+            int2 entry;
+            if (G == 16) {          // one generic load, as fast as a shared one and without a branch
+                entry = *tab;
+                tab += kPerRow;
+            } else if (p.tab_entries) {
+                asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(entry.x), "=r"(entry.y) : "r"(base + L.tab + (c.tab0 + kb * kPerRow + piece) * 8));
+            } else {
+                entry = __ldg(p.tab + c.tab0 + kb * kPerRow + piece);
+            }
+            const int toff = entry.x, tyx = entry.y;
             const int dy = tyx >> 16, dx = static_cast<int16_t>(tyx & 0xffff);
             const uint32_t a0 = base + L.stages + stage * stage_bytes;
             // dy == INT16_MIN: beyond the reduction, meets zero weights whatever it holds
@@ -257,9 +267,9 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
 
     const uint32_t stage_bytes = kBM * kBK + (p.b_res ? 0u : static_cast<uint32_t>(p.b_bytes));
     if (warp >= kEpiWarpsGc && warp < kMmaWarp) {
-        if (p.gran == 16) gather_role<16>(p, L, base, full0, empty0, abort_flag, starve);
-        else if (p.gran == 8) gather_role<8>(p, L, base, full0, empty0, abort_flag, starve);
-        else gather_role<4>(p, L, base, full0, empty0, abort_flag, starve);
+        if (p.gran == 16) gather_role<16>(p, L, sp, base, full0, empty0, abort_flag, starve);
+        else if (p.gran == 8) gather_role<8>(p, L, sp, base, full0, empty0, abort_flag, starve);
+        else gather_role<4>(p, L, sp, base, full0, empty0, abort_flag, starve);
     } else if (warp == kBWarp) {
         if (!p.b_res && lane == 0 && !starve) {
             uint32_t stage = 0, phase = 0;

@@ -1207,8 +1207,8 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         kb_total += c.k_blocks;
         k_pad = std::max(k_pad, c.k_blocks * kBK);
     }
-    p.tab_entries = kb_total * (kBK / p.gran);
-    if (p.tab_entries > 3072) return ENN_B200_INVALID_PARAMS;       // 24 KB of gather table
+    const int32_t tab_total = kb_total * (kBK / p.gran);
+    p.tab_entries = tab_total <= 3072 ? tab_total : 0;      // 24 KB of gather table
     // N tiling: as few tiles as possible (every N tile gathers the A tile again), but split while SMs would idle.
     int32_t tiles_n = (N + max_data - 1) / max_data;
     while (tiles_m * tiles_n < sms && (N + tiles_n) / (tiles_n + 1) >= 32) ++tiles_n;
@@ -1238,7 +1238,10 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     if (b_total > 64 * 1024 || gconv_smem_bytes(p, b_total) > kGcSmemLimit) p.b_res = 0;
     p.stages = 4;
     while (p.stages > 2 && gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) --p.stages;
-    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
+    // Two stages of 256 columns (96 KB) leave room for either 16 KB of constants or a long table, not for both: the constants are then
+    // staged tile by tile, and at last the table stays in global memory (what is left, 96 + 4 + 2 KB and the barriers, always fits).
+    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) p.cols_all = 0;
+    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) p.tab_entries = 0;
     gc->smem_bytes = gconv_smem_bytes(p, p.b_res ? b_total : 0);
     gc->grid = p.n_units < 2 * sms ? p.n_units : 2 * sms;
 
@@ -1246,7 +1249,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     std::vector<ColumnFold> folds(static_cast<size_t>(nc) * N);
     // gather table, then 16 bytes of the input zero point
     const int fill = static_cast<int>((static_cast<uint32_t>(g.in_zp) & 0xff) * 0x01010101u);
-    const size_t fill_at = static_cast<size_t>(p.tab_entries + 1) & ~static_cast<size_t>(1);
+    const size_t fill_at = static_cast<size_t>(tab_total + 1) & ~static_cast<size_t>(1);
     std::vector<int2> tab(fill_at + 2, make_int2(0, INT32_MIN));
     tab[fill_at] = tab[fill_at + 1] = make_int2(fill, fill);
     for (int32_t i = 0; i < nc; ++i) {

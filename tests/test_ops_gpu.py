@@ -1254,6 +1254,11 @@ GCONV_CASES = {
     "deconv_g4_stride3": ("deconv", dict(n=1, h=7, w=6, cin=12, cout=17, k=4, stride=3, pad=1)),
     "deconv_g16_staged": ("deconv", dict(n=5, h=20, w=23, cin=160, cout=136)),
     "deconv_taps_missing": ("deconv", dict(n=1, h=5, w=5, cin=16, cout=8, k=2, stride=3, pad=0)),
+    # two stages of 256 columns fill the shared memory: constants staged tile by tile; tables too long for it, 16- and 4-byte copies
+    "columns_per_tile_1024": ("conv", dict(n=1, h=69, w=70, cin=16, cout=1024, k=3, per_channel=True, out_scale=0.3)),
+    "deconv_columns_per_tile": ("deconv", dict(n=1, h=70, w=71, cin=16, cout=256, k=2, stride=2, pad=0, per_channel=True, out_scale=0.2)),
+    "g16_table_in_global": ("conv", dict(n=1, h=5, w=6, cin=2048, cout=40, k=5, per_channel=True, out_scale=3.0)),
+    "g4_table_in_global": ("conv", dict(n=1, h=6, w=5, cin=508, cout=24, k=5, w_zp=126, out_scale=0.2)),
 }
 
 
