@@ -59,7 +59,7 @@ struct GcParams {
     const int2 *tab;
     const ColParam *cols;       // [class][tiles_n][bn_rows]
     const uint8_t *in;
-    const uint8_t *fill_src;    // 16 bytes of the input zero point
+    const uint8_t *fill_src;    // kBK bytes of the input zero point, a line of their own
     uint8_t *out;
     int64_t out_sn, out_sy, out_sx;
     int32_t *err;

@@ -1247,11 +1247,11 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
 
     std::vector<int8_t> wb(static_cast<size_t>(nc) * tiles_n * p.bn_rows * k_pad, 0);
     std::vector<ColumnFold> folds(static_cast<size_t>(nc) * N);
-    // gather table, then 16 bytes of the input zero point
+    // gather table, then a line of the input zero point
     const int fill = static_cast<int>((static_cast<uint32_t>(g.in_zp) & 0xff) * 0x01010101u);
-    const size_t fill_at = static_cast<size_t>(tab_total + 1) & ~static_cast<size_t>(1);
-    std::vector<int2> tab(fill_at + 2, make_int2(0, INT32_MIN));
-    tab[fill_at] = tab[fill_at + 1] = make_int2(fill, fill);
+    const size_t fill_at = (static_cast<size_t>(tab_total) * sizeof(int2) + kBK - 1) / kBK * (kBK / sizeof(int2));
+    std::vector<int2> tab(fill_at + kBK / sizeof(int2), make_int2(0, INT32_MIN));
+    std::fill(tab.begin() + static_cast<ptrdiff_t>(fill_at), tab.end(), make_int2(fill, fill));
     for (int32_t i = 0; i < nc; ++i) {
         const GcClassDesc &d = classes[i];
         const int32_t K = d.kh * d.kw * cin;
