@@ -67,7 +67,7 @@ __host__ __device__ inline GcSmem gc_smem(const GcParams &p, uint32_t b_res_byte
     s.rows = s.tab + ((static_cast<uint32_t>(p.tab_entries) * 8 + 15) & ~15u);
     s.add = s.rows + kRowTabBytes;
     s.bars = s.add + (p.add_on ? 2048u : 0u);
-    s.total = s.bars + (2 * 8 + 6) * 8 + 16;
+    s.total = s.bars + (2 * kGcMaxStages + 6) * 8 + 16;
     return s;
 }
 
@@ -404,7 +404,7 @@ cudaError_t launch_mode(const GcPlan &plan, cudaStream_t s) {
 }
 template <bool ASUM, int MODE, bool FADD = false>
 cudaError_t set_attr() {
-    return cudaFuncSetAttribute(gconv_kernel<ASUM, MODE, FADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGcSmemLimit);
+    return cudaFuncSetAttribute(gconv_kernel<ASUM, MODE, FADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGcSmemAlone);
 }
 template <bool ASUM>
 cudaError_t set_attrs() {

@@ -76,6 +76,7 @@ struct GcPlan {
     void *w_dev = nullptr, *cols_dev = nullptr, *tab_dev = nullptr;
     size_t smem_bytes = 0;
     int grid = 0;
+    int per_sm = 2;             // CTAs the shared memory is laid out for
     size_t gather_bytes = 0;    // what the matrix would take if it were materialised (limit of the allocation-free call)
 };
 
@@ -86,7 +87,8 @@ struct GcClassDesc {
     int64_t out_base;
 };
 
-constexpr int kGcSmemLimit = 113 * 1024;         // two CTAs per SM
+constexpr uint32_t kGcSmemLimit = 113 * 1024, kGcSmemAlone = 227 * 1024;      // two CTAs per SM, one
+constexpr int kGcMaxStages = 8;
 
 uint32_t gconv_smem_bytes(const GcParams &p, uint32_t b_res_bytes);
 cudaError_t gconv_launch(const GcPlan &plan, cudaStream_t stream);

@@ -1224,7 +1224,18 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         b_tile += tiles_n * p.cls[i].k_blocks;
     }
     p.n_units = unit;
-    p.n_acc = 2 * p.bn_rows <= kMaxBN ? 2 : 1;
+    // CTAs per SM.  Two hide each other's latencies and suit narrow tiles.  Tiles of 256 columns leave them two stages each, on which the
+    // gather and the MMA wait for each other; one CTA has four and a second accumulator.  Measured, a round of unit pairs takes
+    // 1.25 + 0.95 * columns / 256 rounds of single units (64 columns 1.46, 128 1.70, 176 1.9, 256 2.2), so whole rounds decide.  us
+    // with two / with one, 3x3: 128x14x14x512 -> 512 71 / 47, 16x56x56x256 -> 256 40.7 / 28.1, 64x28x28x96 -> 192 17.9 / 13.8;
+    // 32x56x56x128 -> 128 22.0 / 25.8, 256x56x56x64 -> 64 70.9 / 94.8.  Not for 8- and 4-byte gathers (158x27x27x72 -> 184 38.1 / 39.7) and
+    // reductions of one or two k-blocks, whose time is the epilogue's.
+    {
+        const int64_t single = (p.n_units + sms - 1) / sms, pairs = (p.n_units + 2 * sms - 1) / (2 * sms);
+        const bool alone = p.n_units > sms && p.gran == 16 && kb_total > 2 * nc && single * 256 * 100 < pairs * (125 * 256 + 95 * p.bn_rows);
+        gc->per_sm = ctx->has_opt("gc_per_sm") ? (ctx->opt("gc_per_sm") == 1 ? 1 : 2) : (alone ? 1 : 2);
+    }
+    p.n_acc = gc->per_sm == 1 || 2 * p.bn_rows <= kMaxBN ? 2 : 1;      // half of the 512 columns per CTA, or all of them
     p.tmem_cols = 32;
     while (p.tmem_cols < p.n_acc * p.bn_rows) p.tmem_cols *= 2;
     p.idesc = (2u << 4) | (static_cast<uint32_t>(g.a_signed ? 1 : 0) << 7) | (1u << 10) | (static_cast<uint32_t>(p.bn_rows >> 3) << 17) |
@@ -1232,18 +1243,19 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     p.b_bytes = p.bn_rows * kBK;
     p.cols_all = nc * tiles_n * p.bn_rows <= 1024;      // 16 KB
     // Weights stay in shared memory where three stages of A fit beside them, else they travel with the stages.
-    const uint32_t b_total = static_cast<uint32_t>(std::min<int64_t>(static_cast<int64_t>(b_tile) * p.b_bytes, 1 << 20));
+    const uint32_t limit = gc->per_sm == 1 ? kGcSmemAlone : kGcSmemLimit;
+    uint32_t b_res_bytes = static_cast<uint32_t>(std::min<int64_t>(static_cast<int64_t>(b_tile) * p.b_bytes, 1 << 20));
     p.b_res = 1;
     p.stages = 3;
-    if (b_total > 64 * 1024 || gconv_smem_bytes(p, b_total) > kGcSmemLimit) p.b_res = 0;
-    p.stages = 4;
-    while (p.stages > 2 && gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) --p.stages;
+    if (b_res_bytes > (gc->per_sm == 1 ? 128u : 64u) * 1024 || gconv_smem_bytes(p, b_res_bytes) > limit) p.b_res = 0, b_res_bytes = 0;
+    p.stages = gc->per_sm == 1 ? kGcMaxStages : 4;
+    while (p.stages > 2 && gconv_smem_bytes(p, b_res_bytes) > limit) --p.stages;
     // Two stages of 256 columns (96 KB) leave room for either 16 KB of constants or a long table, not for both: the constants are then
     // staged tile by tile, and at last the table stays in global memory (what is left, 96 + 4 + 2 KB and the barriers, always fits).
-    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) p.cols_all = 0;
-    if (gconv_smem_bytes(p, p.b_res ? b_total : 0) > kGcSmemLimit) p.tab_entries = 0;
-    gc->smem_bytes = gconv_smem_bytes(p, p.b_res ? b_total : 0);
-    gc->grid = p.n_units < 2 * sms ? p.n_units : 2 * sms;
+    if (gconv_smem_bytes(p, b_res_bytes) > limit) p.cols_all = 0;
+    if (gconv_smem_bytes(p, b_res_bytes) > limit) p.tab_entries = 0;
+    gc->smem_bytes = std::max<size_t>(gconv_smem_bytes(p, b_res_bytes), gc->per_sm == 1 ? kGcSmemLimit + 2048 : 0);
+    gc->grid = std::min(p.n_units, gc->per_sm * sms);
 
     std::vector<int8_t> wb(static_cast<size_t>(nc) * tiles_n * p.bn_rows * k_pad, 0);
     std::vector<ColumnFold> folds(static_cast<size_t>(nc) * N);

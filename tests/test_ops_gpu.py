@@ -1259,6 +1259,10 @@ GCONV_CASES = {
     "deconv_columns_per_tile": ("deconv", dict(n=1, h=70, w=71, cin=16, cout=256, k=2, stride=2, pad=0, per_channel=True, out_scale=0.2)),
     "g16_table_in_global": ("conv", dict(n=1, h=5, w=6, cin=2048, cout=40, k=5, per_channel=True, out_scale=3.0)),
     "g4_table_in_global": ("conv", dict(n=1, h=6, w=5, cin=508, cout=24, k=5, w_zp=126, out_scale=0.2)),
+    # one CTA per SM (two accumulators of 256 columns, more than one round of units): weights resident, travelling, two N tiles
+    "alone_resident": ("conv", dict(n=1, h=139, w=140, cin=48, cout=250, k=3, per_channel=True, out_scale=0.4)),
+    "alone_staged_asum": ("conv", dict(n=1, h=140, w=139, cin=64, cout=240, k=3, w_zp=119, out_scale=0.05)),
+    "alone_two_tiles": ("conv", dict(n=1, h=97, w=98, cin=32, cout=500, k=3, per_channel=True, out_scale=0.4, act=cases.enn.ACT_NONE)),
 }
 
 
