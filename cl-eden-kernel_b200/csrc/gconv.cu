@@ -11,7 +11,7 @@
 // Why a gather by ordinary threads and not tensor copies: a tensor copy of an im2col tile costs several cycles per pixel row
 // whatever the row's length (a 3x3 layer over 64 channels fetches nine 64-byte rows per output pixel), cannot fill borders
 // with a zero point other than 0, and needs rows whose pitch is a multiple of 16 bytes.  The threads address any geometry
-// through a table of (byte offset, dy, dx) per copy, the nine-fold re-reads of a 3x3 window hit the L1, the reduction is
+// through a table of (offset, dy, dx) per copy, the nine-fold re-reads of a 3x3 window hit the L1, the reduction is
 // packed densely (tap-major, no padding per tap) and no zero-point padded or gathered copy of the input is written first.
 //
 // Every wait is bounded (tc_common.cuh): on expiry an error code reaches the host and all roles fall through to the exit.
@@ -26,7 +26,7 @@ constexpr int kEpiWarpsGc = 4, kGatherWarps = 4;
 constexpr int kGatherThreads = 32 * kGatherWarps;
 constexpr int kMmaWarp = kEpiWarpsGc + kGatherWarps, kBWarp = kMmaWarp + 1;
 constexpr int kGcThreads = 32 * (kBWarp + 1);
-constexpr int kRowTabBytes = kBM * 16;          // {byte offset, iy, ix, -} of the 32 rows each gather warp fetches
+constexpr int kRowTabBytes = kBM * 16;          // {64-bit address, iy, ix} of the 32 rows each gather warp fetches
 
 template <int OFF>
 __device__ __forceinline__ void cp_async16(uint32_t dst, const uint8_t *src) {
@@ -43,6 +43,12 @@ __device__ __forceinline__ void st_shared(uint32_t dst, const uint2 &v) {
 template <int OFF>
 __device__ __forceinline__ void st_shared(uint32_t dst, uint32_t v) {
     asm volatile("st.shared.b32 [%0 + %2], %1;" ::"r"(dst), "r"(v), "n"(OFF) : "memory");
+}
+// One entry of the row table.
+__device__ __forceinline__ void load_row(uint32_t addr, const uint8_t *&row, int &iy, int &ix) {
+    uint32_t lo, hi;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(lo), "=r"(hi), "=r"(iy), "=r"(ix) : "r"(addr));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(row) : "r"(lo), "r"(hi));
 }
 // f(integral_constant<int, i>) for i = 0 .. N - 1, unrolled.
 template <int I, int N, typename F>
@@ -135,24 +141,23 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
         {
             const int r = wbase + lane % kRowsPerWarp + kRowsPerPass * (lane / kRowsPerWarp);
             const uint32_t m = static_cast<uint32_t>(u.tm * kBM + r);
-            int off = 0, iy = -(1 << 20), ix = 0;
+            const uint8_t *row = in;                // 64-bit: an input may be larger than 4 GiB
+            int iy = INT32_MIN / 2, ix = 0;         // rows beyond the class: outside whatever the tap
             if (m < static_cast<uint32_t>(c.M)) {
                 const uint32_t img = c.div_img.div(m), rem = m - img * static_cast<uint32_t>(c.oh * c.ow);
                 const uint32_t oy = c.div_ow.div(rem), ox = rem - oy * static_cast<uint32_t>(c.ow);
                 iy = static_cast<int>(oy) * p.sy + c.y0;
                 ix = static_cast<int>(ox) * p.sx + c.x0;
-                off = ((static_cast<int>(img) * p.h + iy) * p.w + ix) * p.cin;
+                row += ((static_cast<int64_t>(img) * p.h + iy) * p.w + ix) * p.cin;
             }
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rt + lane * 16), "r"(off), "r"(iy), "r"(ix), "r"(0) : "memory");
+            asm volatile("st.shared.b64 [%0], %1;\n\tst.shared.v2.b32 [%0 + 8], {%2, %3};" ::"r"(rt + lane * 16), "l"(row), "r"(iy), "r"(ix) : "memory");
         }
         __syncwarp();
-        int roff[G == 16 ? kPasses : 1], riy[G == 16 ? kPasses : 1], rix[G == 16 ? kPasses : 1];
+        const uint8_t *rrow[G == 16 ? kPasses : 1];
+        int riy[G == 16 ? kPasses : 1], rix[G == 16 ? kPasses : 1];
         if (G == 16) {
 #pragma unroll
-            for (int i = 0; i < kPasses; ++i) {
-                int pad;
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(roff[i]), "=r"(riy[i]), "=r"(rix[i]), "=r"(pad) : "r"(rt_lane + i * kRowsPerWarp * 16));
-            }
+            for (int i = 0; i < kPasses; ++i) load_row(rt_lane + i * kRowsPerWarp * 16, rrow[i], riy[i], rix[i]);
         }
         const int2 *tab = tab0 + c.tab0;
         for (int kb = 0; kb < c.k_blocks; ++kb) {
@@ -177,7 +182,7 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                     static_for<0, kPasses>([&](auto tag) {
                         constexpr int i = decltype(tag)::value;
                         const bool inside = static_cast<uint32_t>(riy[i] + dy) < h && static_cast<uint32_t>(rix[i] + dx) < w;
-                        cp_async16<i * kRowsPerPass * kBK>(a0 + dst0, inside ? in + static_cast<uint32_t>(roff[i] + toff) : fill_src);
+                        cp_async16<i * kRowsPerPass * kBK>(a0 + dst0, inside ? rrow[i] + toff : fill_src);
                     });
                 cp_async_arrive(full0 + 8 * stage);
             } else {
@@ -186,11 +191,11 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                 if (dy != INT16_MIN) {
                     static_for<0, kPasses>([&](auto tag) {
                         constexpr int i = decltype(tag)::value;
-                        int off, iy, ix, pad;
-                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4 + %5];" : "=r"(off), "=r"(iy), "=r"(ix), "=r"(pad)
-                                     : "r"(rt_lane), "n"(i * kRowsPerWarp * 16));
+                        const uint8_t *row;
+                        int iy, ix;
+                        load_row(rt_lane + i * kRowsPerWarp * 16, row, iy, ix);
                         const bool inside = static_cast<uint32_t>(iy + dy) < h && static_cast<uint32_t>(ix + dx) < w;
-                        v[i] = __ldg(reinterpret_cast<const Word *>(inside ? in + static_cast<uint32_t>(off + toff) : fill_src));
+                        v[i] = __ldg(reinterpret_cast<const Word *>(inside ? row + toff : fill_src));
                     });
                     static_for<0, kPasses>([&](auto tag) {
                         constexpr int i = decltype(tag)::value;

@@ -56,7 +56,7 @@ struct GcParams {
     int32_t need_asum, zw_eff, a_signed, act_min, act_max, out_zp, mode, sat_plain;
     uint32_t idesc;
     int32_t h, w, cin, sy, sx;
-    const int2 *tab;
+    const int2 *tab;            // {byte offset from the row's first position, dy << 16 | dx}
     const ColParam *cols;       // [class][tiles_n][bn_rows]
     const uint8_t *in;
     const uint8_t *fill_src;    // kBK bytes of the input zero point, a line of their own

@@ -1172,7 +1172,6 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
                     int64_t out_sn, int64_t out_sy, int64_t out_sx, WeightFn weight, GcPlan *gc) {
     const int32_t N = g.cout, cin = g.cin, nc = static_cast<int32_t>(classes.size());
     if (nc < 1 || nc > kGcMaxClasses || (cin & 3) != 0) return ENN_B200_INVALID_PARAMS;
-    if (static_cast<int64_t>(g.n) * g.h * g.w * cin >= (1ll << 31) - (1 << 20)) return ENN_B200_INVALID_PARAMS;      // 32-bit byte offsets
     GcParams &p = gc->prm;
     p.n_classes = nc;
     p.N = N;

@@ -1293,3 +1293,28 @@ def test_gather_convolution(enn, orc, ctx, name):
         _check(op, y_ref, x)
     finally:
         op.release()
+
+
+def test_gather_convolution_beyond_2_gib(enn, orc, ctx):
+    """Byte offsets past 2^31: images on both sides of the boundary and the last one against the oracle (the others hold whatever)."""
+    n, h, w, cin, cout = 680, 224, 224, 64, 16
+    pixels = h * w
+    d, x, wt, b, sc = cases.conv_case(seed=91, n=3, h=h, w=w, cin=cin, cout=cout, k=3, w_zp=121, out_scale=0.05)
+    first_past = (1 << 31) // (pixels * cin)
+    d.n = 1
+    want = [orc.conv2d(d, x[i:i + 1], wt, b, sc).reshape(-1) for i in range(3)]
+    d.n = n
+    op = enn.conv2d(ctx, d, wt, b, sc)
+    a, o = ctx.malloc(n * pixels * cin), ctx.malloc(n * pixels * cout)
+    try:
+        assert op.info.impl == enn.IMPL_TCGEN05 and op.info.kernel_launches == 1
+        where = (0, first_past, n - 1)
+        for img, xi in zip(where, x):
+            ctx.upload(type(a)(a.value + img * pixels * cin), xi)
+        op.execute(a, o)
+        for img, y in zip(where, want):
+            assert np.array_equal(ctx.download(type(o)(o.value + img * pixels * cout), (pixels * cout,)), y)
+    finally:
+        ctx.free(a)
+        ctx.free(o)
+        op.release()
