@@ -1190,7 +1190,8 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         const GcClassDesc &d = classes[i];
         const int64_t M = static_cast<int64_t>(g.n) * d.oh * d.ow, K = static_cast<int64_t>(d.kh) * d.kw * cin;
         if (M <= 0 || M > INT32_MAX - kBM || K > (1 << 20)) return ENN_B200_INVALID_PARAMS;
-        if ((d.kh - 1) * std::abs(d.dy) >= 32000 || (d.kw - 1) * std::abs(d.dx) >= 32000 || g.h >= 32000 || g.w >= 32000) return ENN_B200_INVALID_PARAMS;
+        // a tap's displacement is kept in 16 bits; the image itself may be of any size
+        if (static_cast<int64_t>(d.kh - 1) * std::abs(d.dy) >= 32000 || static_cast<int64_t>(d.kw - 1) * std::abs(d.dx) >= 32000) return ENN_B200_INVALID_PARAMS;
         GcClass &c = p.cls[i];
         c.M = static_cast<int32_t>(M);
         c.tiles_m = static_cast<int32_t>((M + kBM - 1) / kBM);

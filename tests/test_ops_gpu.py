@@ -1262,6 +1262,9 @@ GCONV_CASES = {
     # one CTA per SM (two accumulators of 256 columns, more than one round of units): weights resident, travelling, two N tiles
     "alone_resident": ("conv", dict(n=1, h=139, w=140, cin=48, cout=250, k=3, per_channel=True, out_scale=0.4)),
     "alone_staged_asum": ("conv", dict(n=1, h=140, w=139, cin=64, cout=240, k=3, w_zp=119, out_scale=0.05)),
+    "sequence": ("conv", dict(n=2, h=1, w=40001, cin=32, cout=24, kh=1, kw=5, per_channel=True, out_scale=0.2)),
+    "tall_dilated": ("conv", dict(n=1, h=33000, w=2, cin=16, cout=16, k=3, dil=7, stride=2, w_zp=140, out_scale=0.05)),
+    "deconv_sequence": ("deconv", dict(n=1, h=32768, w=1, cin=32, cout=16, k=4)),
     "alone_two_tiles": ("conv", dict(n=1, h=97, w=98, cin=32, cout=500, k=3, per_channel=True, out_scale=0.4, act=cases.enn.ACT_NONE)),
 }
 
