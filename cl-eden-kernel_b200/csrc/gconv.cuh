@@ -1,4 +1,4 @@
-// Gather convolution: one launch for every dense contraction whose A operand cannot be read in place (taps, strides,
+// Gather convolution: one launch (transposed convolutions of stride 4 and more: several) for every dense contraction whose A operand cannot be read in place (taps, strides,
 // dilation, zero-point borders, rows whose byte pitch is no multiple of 16, the parity classes of a transposed convolution).
 #pragma once
 #include <cuda.h>
@@ -10,7 +10,7 @@
 
 namespace enn_b200 {
 
-constexpr int kGcMaxClasses = 9;
+constexpr int kGcMaxClasses = 9;        // of one launch: strides up to 3
 
 // Quotient by an invariant divisor for dividends below 2^31: q = umulhi(n, mul) >> shift, with mul = ceil(2^(31 + s) / d) and
 // shift = s - 1 for s = ceil(log2 d), d > 1 (Granlund and Montgomery, "Division by invariant integers using

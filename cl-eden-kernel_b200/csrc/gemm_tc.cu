@@ -999,7 +999,9 @@ struct TcPlan {
     std::vector<TcGemm> gemms;
     void *scratch = nullptr;           // im2col matrix, shared by the GEMMs of the op (they run in stream order)
     size_t scratch_bytes = 0;
-    std::unique_ptr<GcPlan> gc;        // gather convolution (gconv.cu): replaces the list of GEMMs
+    // Gather convolution (gconv.cu), which replaces the list of GEMMs: one launch, or one per kGcMaxClasses parity classes of a
+    // transposed convolution.
+    std::vector<std::unique_ptr<GcPlan>> gcs;
     int32_t *err_host = nullptr;       // pinned + mapped
     int32_t *err_dev = nullptr;
     bool starve_next = false;          // the next execute runs the bounded-wait self-test (tc_test_starve_next)
@@ -1321,6 +1323,15 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     return ENN_B200_SUCCESS;
 }
 
+void free_gconvs(TcPlan *plan) {
+    for (auto &gc : plan->gcs) {
+        if (gc->w_dev) cudaFree(gc->w_dev);
+        if (gc->cols_dev) cudaFree(gc->cols_dev);
+        if (gc->tab_dev) cudaFree(gc->tab_dev);
+    }
+    plan->gcs.clear();
+}
+
 void free_plan(TcPlan *plan) {
     if (!plan) return;
     for (auto &gm : plan->gemms) {
@@ -1328,11 +1339,7 @@ void free_plan(TcPlan *plan) {
         if (gm.cols_dev) cudaFree(gm.cols_dev);
         if (gm.ktab_dev) cudaFree(gm.ktab_dev);
     }
-    if (plan->gc) {
-        if (plan->gc->w_dev) cudaFree(plan->gc->w_dev);
-        if (plan->gc->cols_dev) cudaFree(plan->gc->cols_dev);
-        if (plan->gc->tab_dev) cudaFree(plan->gc->tab_dev);
-    }
+    free_gconvs(plan);
     if (plan->scratch) cudaFree(plan->scratch);
     if (plan->err_host) cudaFreeHost(plan->err_host);
     delete plan;
@@ -1481,17 +1488,26 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         return ENN_B200_SUCCESS;
     };
 
-    // Plans the operator as one gather convolution; on success the plan is complete.
+    // Plans the operator as a gather convolution; on success the plan is complete.  The classes are spread evenly over as few launches
+    // as hold them (transposed convolutions of stride 4: 16 classes in two launches).
     auto try_gconv = [&](const std::vector<GcClassDesc> &classes, int32_t sy, int32_t sx, int64_t sn, int64_t s_y, int64_t s_x, auto wfn) -> int32_t {
-        std::unique_ptr<GcPlan> gc(new (std::nothrow) GcPlan());
-        if (!gc) return bail(ENN_B200_FAILURE);
-        plan->gc = std::move(gc);
-        const int32_t s2 = build_gconv(ctx, g, qh, classes, sy, sx, sn, s_y, s_x, wfn, plan->gc.get());
-        if (s2 == ENN_B200_INVALID_PARAMS) {
-            plan->gc.reset();       // nothing was allocated
-            return s2;
+        const int32_t nc = static_cast<int32_t>(classes.size()), launches = (nc + kGcMaxClasses - 1) / kGcMaxClasses;
+        if (nc == 0) return ENN_B200_INVALID_PARAMS;
+        for (int32_t l = 0; l < launches; ++l) {
+            const int32_t c0 = static_cast<int32_t>(static_cast<int64_t>(nc) * l / launches), c1 = static_cast<int32_t>(static_cast<int64_t>(nc) * (l + 1) / launches);
+            plan->gcs.emplace_back(new (std::nothrow) GcPlan());
+            if (!plan->gcs.back()) {
+                plan->gcs.pop_back();
+                return bail(ENN_B200_FAILURE);
+            }
+            const int32_t s2 = build_gconv(ctx, g, qh, std::vector<GcClassDesc>(classes.begin() + c0, classes.begin() + c1), sy, sx, sn, s_y, s_x,
+                                           [&](int32_t i, int32_t n, int32_t k) { return wfn(c0 + i, n, k); }, plan->gcs.back().get());
+            if (s2 == ENN_B200_INVALID_PARAMS) {
+                free_gconvs(plan);
+                return s2;
+            }
+            if (s2 != ENN_B200_SUCCESS) return bail(s2);
         }
-        if (s2 != ENN_B200_SUCCESS) return bail(s2);
         plan->gemms.clear();
         if (cudaHostAlloc(reinterpret_cast<void **>(&plan->err_host), sizeof(int32_t), cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer(reinterpret_cast<void **>(&plan->err_dev), plan->err_host, 0) != cudaSuccess) {
@@ -1499,8 +1515,8 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             return bail(ENN_B200_CUDA_FAILURE);
         }
         *plan->err_host = 0;
-        plan->gc->prm.err = plan->err_dev;
-        op->info.kernel_launches = 1;
+        for (auto &gc : plan->gcs) gc->prm.err = plan->err_dev;
+        op->info.kernel_launches = launches;
         op->tc = plan;
         return ENN_B200_SUCCESS;
     };
@@ -1744,12 +1760,13 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
 // INVALID_PARAMS when this plan cannot take it; the caller then keeps the two operators.
 int32_t tc_fuse_add(enn_b200_op *op, const AddParams &add, bool conv_is_second) {
     TcPlan *plan = static_cast<TcPlan *>(op->tc);
-    if (plan && plan->gc && !plan->fused_add) {
-        GcParams &p = plan->gc->prm;
+    if (plan && !plan->gcs.empty() && !plan->fused_add) {
+        GcPlan &gc = *plan->gcs[0];         // a convolution is one launch
+        GcParams &p = gc.prm;
         if (op->kind != OP_CONV || (p.mode != kModeNudge && p.mode != kModeGeneral) || (p.N & 15) != 0 || !add.lut || add.is_signed != p.a_signed)
             return ENN_B200_INVALID_PARAMS;
-        if (plan->gc->smem_bytes + 2048 > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
-        plan->gc->smem_bytes += 2048;
+        if (gc.smem_bytes + 2048 > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
+        gc.smem_bytes += 2048;
         p.add = add;
         p.add_on = 1;
         p.add_swap = conv_is_second ? 1 : 0;
@@ -1780,8 +1797,7 @@ void tc_set_residual(enn_b200_op *op, const void *res) {
 namespace {
 int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) {
     enn_b200_context *ctx = op->ctx;
-    GcParams &p = plan->gc->prm;
-    if ((reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(p.gran - 1)) != 0) {
+    if ((reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(plan->gcs[0]->prm.gran - 1)) != 0) {
         // sub-buffers at odd offsets: the general kernels take any alignment
         if (plan->fused_add) {
             ctx->last_error = "fused convolution + add needs 16-byte aligned pointers";
@@ -1798,16 +1814,22 @@ int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) 
             ctx->last_error = "fused convolution + add needs the second addend and 16-byte aligned pointers";
             return ENN_B200_INVALID_PARAMS;
         }
-        p.add_res = plan->residual;
     }
-    p.in = static_cast<const uint8_t *>(in);
-    p.out = static_cast<uint8_t *>(out);
-    p.test_starve = plan->starve_next ? 1 : 0;
+    const bool starve = plan->starve_next;
     plan->starve_next = false;
-    const cudaError_t e = gconv_launch(*plan->gc, ctx->stream);
-    if (e == cudaSuccess) return ENN_B200_SUCCESS;
-    ctx->last_error = std::string("gconv_kernel launch: ") + cudaGetErrorString(e);
-    return ENN_B200_CUDA_FAILURE;
+    for (auto &gc : plan->gcs) {
+        GcParams &p = gc->prm;
+        p.in = static_cast<const uint8_t *>(in);
+        p.out = static_cast<uint8_t *>(out);
+        p.add_res = plan->fused_add ? plan->residual : nullptr;
+        p.test_starve = starve ? 1 : 0;
+        const cudaError_t e = gconv_launch(*gc, ctx->stream);
+        if (e != cudaSuccess) {
+            ctx->last_error = std::string("gconv_kernel launch: ") + cudaGetErrorString(e);
+            return ENN_B200_CUDA_FAILURE;
+        }
+    }
+    return ENN_B200_SUCCESS;
 }
 }  // namespace
 
@@ -1821,7 +1843,7 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = buf;
         return ENN_B200_CUDA_FAILURE;
     }
-    if (plan->gc) return gconv_execute(op, plan, in, out);
+    if (!plan->gcs.empty()) return gconv_execute(op, plan, in, out);
     const bool starve = plan->starve_next;
     plan->starve_next = false;
     for (auto &gm : plan->gemms) {
@@ -1952,7 +1974,8 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = "enn_b200_op_execute_noalloc: the operator is not bound to the tensor-core path (or has a fused add)";
         return ENN_B200_INVALID_PARAMS;
     }
-    size_t need = plan->gc ? plan->gc->gather_bytes : 0;
+    size_t need = 0;
+    for (auto &gc : plan->gcs) need = std::max(need, gc->gather_bytes);
     for (auto &gm : plan->gemms) {
         if (!gm.gather) {
             ctx->last_error = "enn_b200_op_execute_noalloc: this operator has no gathered input matrix; call enn_b200_op_execute";
@@ -1968,7 +1991,7 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = buf;
         return ENN_B200_INVALID_PARAMS;
     }
-    if (plan->gc) {      // gathers into shared memory: no scratch array needed
+    if (!plan->gcs.empty()) {      // gathers into shared memory: no scratch array needed
         if (*plan->err_host == 0) return gconv_execute(op, plan, in, out);
         ctx->last_error = "gather convolution gave up on a barrier wait earlier";
         return ENN_B200_CUDA_FAILURE;

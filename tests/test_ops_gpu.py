@@ -1298,6 +1298,23 @@ def test_gather_convolution(enn, orc, ctx, name):
         op.release()
 
 
+@pytest.mark.parametrize("launches,kw", [
+    (2, dict(n=2, h=9, w=7, cin=32, cout=24, k=8, stride=4, pad=2, per_channel=True, out_scale=0.3)),
+    (2, dict(n=1, h=5, w=6, cin=20, cout=33, k=4, stride=4, pad=0)),
+    (3, dict(n=1, h=4, w=5, cin=16, cout=8, k=3, stride=5, pad=0)),              # parity classes without taps
+    (8, dict(n=1, h=3, w=4, cin=64, cout=21, k=16, stride=8, pad=4)),
+])
+def test_gather_deconvolution_many_classes(enn, orc, ctx, launches, kw):
+    """Strides above 3 have more parity classes than one launch takes."""
+    d, x, w, b, sc = cases.deconv_case(seed=92, **kw)
+    op = enn.deconv(ctx, d, w, b, sc)
+    try:
+        assert op.info.impl == enn.IMPL_TCGEN05 and op.info.kernel_launches == launches
+        _check(op, orc.deconv(d, x, w, b, sc), x)
+    finally:
+        op.release()
+
+
 def test_gather_convolution_beyond_2_gib(enn, orc, ctx):
     """Byte offsets past 2^31: images on both sides of the boundary and the last one against the oracle (the others hold whatever)."""
     n, h, w, cin, cout = 680, 224, 224, 64, 16
