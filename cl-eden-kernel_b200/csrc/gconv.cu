@@ -107,7 +107,8 @@ struct UnitWalk {
 //            every copy in flight (about 1000 cycles per k-block, measured).
 //   G < 16   8- or 4-byte loads into registers, all of a k-block in flight, then stores, fence, one arrival per warp.
 //            Asynchronous copies of 8 bytes took 27 SM cycles per warp instruction (16 bytes: 10), loads and stores 4 to 6.
-template <int G>
+//   BYTES    4-byte words put together from single bytes: inputs at odd addresses.
+template <int G, bool BYTES = false>
 __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, const uint8_t *sp, uint32_t base, uint32_t full0, uint32_t empty0,
                                             volatile int *abort_flag, bool starve) {
     constexpr int kPerRow = kBK / G;                            // copies per A row and k-block: 8, 16 or 32
@@ -124,14 +125,17 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
     // A row's lanes copy a border position from the line of zero points each at its own place, as they would an inside one: lanes that
     // all copied the same 16 bytes were served one after another (1x28x28x512 -> 512, whose last M tile has 16 real rows of 128:
     // 31.2 -> 15.1 us; 1x56x56x64 -> 64 5.9 -> 4.6; 256x56x56x64 -> 64 72.3 -> 70.9).
-    const uint8_t *in = p.in, *fill_src = p.fill_src + piece * G;
+    // A copy smaller than a table entry's unit reads the entry of its unit, a few bytes further on.
+    const int unit_log2 = G == 16 ? 4 : p.unit_log2, per_kb = kBK >> unit_log2;
+    const int first = (piece * G) >> unit_log2, sub = (piece * G) & ((1 << unit_log2) - 1);
+    const uint8_t *fill_src = p.fill_src + piece * G;
     const uint32_t h = static_cast<uint32_t>(p.h), w = static_cast<uint32_t>(p.w);
     const uint32_t stage_bytes = kBM * kBK + (p.b_res ? 0u : static_cast<uint32_t>(p.b_bytes));
     // A warp fetches kRowsPerWarp rows per pass, 32 rows per tile: the lanes work them out and leave them in the warp's table.
     constexpr int kRowsPerWarp = 32 / kPerRow;                  // 4, 2 or 1
     const int wbase = (t >> 5) * kRowsPerWarp;
     const uint32_t rt = base + L.rows + static_cast<uint32_t>(t >> 5) * 512u, rt_lane = rt + static_cast<uint32_t>(lane / kPerRow) * 16;
-    const int2 *const tab0 = (p.tab_entries ? reinterpret_cast<const int2 *>(sp + L.tab) : p.tab) + piece;
+    const int2 *const tab0 = (p.tab_entries ? reinterpret_cast<const int2 *>(sp + L.tab) : p.tab) + first;
     uint32_t stage = 0, phase = 0;
     bool ok = !starve;
     UnitWalk u;
@@ -141,7 +145,7 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
         {
             const int r = wbase + lane % kRowsPerWarp + kRowsPerPass * (lane / kRowsPerWarp);
             const uint32_t m = static_cast<uint32_t>(u.tm * kBM + r);
-            const uint8_t *row = in;                // 64-bit: an input may be larger than 4 GiB
+            const uint8_t *row = p.in;              // 64-bit: an input may be larger than 4 GiB
             int iy = INT32_MIN / 2, ix = 0;         // rows beyond the class: outside whatever the tap
             if (m < static_cast<uint32_t>(c.M)) {
                 const uint32_t img = c.div_img.div(m), rem = m - img * static_cast<uint32_t>(c.oh * c.ow);
@@ -162,11 +166,11 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
         const int2 *tab = tab0 + c.tab0;
         for (int kb = 0; kb < c.k_blocks; ++kb) {
             const int2 entry = *tab;        // ahead of the wait, which hides the load (7x7 over 8x14x14x1024, 392 k-blocks: 178 -> 138 us)
-            tab += kPerRow;
+            tab += per_kb;
             if (lane == 0) ok = mbar_test_wait(empty0 + 8 * stage, phase ^ 1) || mbar_wait_fast(empty0 + 8 * stage, phase ^ 1, abort_flag, p.err, 1);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
-            const int toff = entry.x, tyx = entry.y;
+            const int toff = entry.x + sub, tyx = entry.y;
             const int dy = tyx >> 16, dx = static_cast<int16_t>(tyx & 0xffff);
             const uint32_t a0 = base + L.stages + stage * stage_bytes;
             // dy == INT16_MIN: beyond the reduction, meets zero weights whatever it holds
@@ -180,21 +184,41 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                 cp_async_arrive(full0 + 8 * stage);
             } else {
                 using Word = std::conditional_t<G == 8, uint2, uint32_t>;
-                Word v[kPasses];
+                constexpr int kPart = BYTES ? 8 : kPasses;      // loads in flight: all of the k-block, or what the registers hold
                 if (dy != INT16_MIN) {
-                    static_for<0, kPasses>([&](auto tag) {
-                        constexpr int i = decltype(tag)::value;
-                        const uint8_t *row;
-                        int iy, ix;
-                        load_row(rt_lane + i * kRowsPerWarp * 16, row, iy, ix);
-                        const bool inside = static_cast<uint32_t>(iy + dy) < h && static_cast<uint32_t>(ix + dx) < w;
-                        v[i] = __ldg(reinterpret_cast<const Word *>(inside ? row + toff : fill_src));
-                    });
-                    static_for<0, kPasses>([&](auto tag) {
-                        constexpr int i = decltype(tag)::value;
-                        if constexpr (kRowsPerPass == 4) st_shared<(i & ~1) * kRowsPerPass * kBK>(a0 + (i & 1 ? dst1 : dst0), v[i]);
-                        else st_shared<i * kRowsPerPass * kBK>(a0 + dst0, v[i]);
-                    });
+                    if constexpr (BYTES) {
+#pragma unroll 1
+                        for (int part = 0; part < kPasses; part += kPart) {
+                            Word v[kPart];
+#pragma unroll
+                            for (int i = 0; i < kPart; ++i) {
+                                const uint8_t *row;
+                                int iy, ix;
+                                load_row(rt_lane + (part + i) * kRowsPerWarp * 16, row, iy, ix);
+                                const bool inside = static_cast<uint32_t>(iy + dy) < h && static_cast<uint32_t>(ix + dx) < w;
+                                const uint8_t *src = inside ? row + toff : fill_src;
+                                v[i] = __ldg(src) | __ldg(src + 1) << 8 | __ldg(src + 2) << 16 | static_cast<uint32_t>(__ldg(src + 3)) << 24;
+                            }
+#pragma unroll
+                            for (int i = 0; i < kPart; ++i)
+                                st_shared<0>(a0 + (i & 1 ? dst1 : dst0) + static_cast<uint32_t>(part + (i & ~1)) * kRowsPerPass * kBK, v[i]);
+                        }
+                    } else {
+                        Word v[kPasses];
+                        static_for<0, kPasses>([&](auto tag) {
+                            constexpr int i = decltype(tag)::value;
+                            const uint8_t *row;
+                            int iy, ix;
+                            load_row(rt_lane + i * kRowsPerWarp * 16, row, iy, ix);
+                            const bool inside = static_cast<uint32_t>(iy + dy) < h && static_cast<uint32_t>(ix + dx) < w;
+                            v[i] = __ldg(reinterpret_cast<const Word *>(inside ? row + toff : fill_src));
+                        });
+                        static_for<0, kPasses>([&](auto tag) {
+                            constexpr int i = decltype(tag)::value;
+                            if constexpr (kRowsPerPass == 4) st_shared<(i & ~1) * kRowsPerPass * kBK>(a0 + (i & 1 ? dst1 : dst0), v[i]);
+                            else st_shared<i * kRowsPerPass * kBK>(a0 + dst0, v[i]);
+                        });
+                    }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
@@ -270,7 +294,8 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
     if (warp >= kEpiWarpsGc && warp < kMmaWarp) {
         if (p.gran == 16) gather_role<16>(p, L, sp, base, full0, empty0, abort_flag, starve);
         else if (p.gran == 8) gather_role<8>(p, L, sp, base, full0, empty0, abort_flag, starve);
-        else gather_role<4>(p, L, sp, base, full0, empty0, abort_flag, starve);
+        else if (p.gran == 4) gather_role<4>(p, L, sp, base, full0, empty0, abort_flag, starve);
+        else gather_role<4, true>(p, L, sp, base, full0, empty0, abort_flag, starve);
     } else if (warp == kBWarp) {
         if (!p.b_res && lane == 0 && !starve) {
             uint32_t stage = 0, phase = 0;
@@ -387,7 +412,8 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
 
 template <bool ASUM, int MODE, bool FADD = false>
 cudaError_t launch_one(const GcPlan &plan, cudaStream_t s) {
-    return launch_pdl(gconv_kernel<ASUM, MODE, FADD>, dim3(static_cast<unsigned>(plan.grid)), dim3(kGcThreads), plan.smem_bytes, s, plan.map_b, plan.prm);
+    return launch_pdl(gconv_kernel<ASUM, MODE, FADD>,
+                      dim3(static_cast<unsigned>(plan.grid)), dim3(kGcThreads), plan.smem_bytes, s, plan.map_b, plan.prm);
 }
 template <bool ASUM>
 cudaError_t launch_mode(const GcPlan &plan, cudaStream_t s) {

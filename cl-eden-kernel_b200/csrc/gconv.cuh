@@ -50,8 +50,9 @@ struct GcParams {
     int32_t tmem_cols;
     int32_t b_res;              // all weights stay in shared memory
     int32_t b_bytes;            // one (N tile, k-block) of weights
-    int32_t tab_entries;        // gather table entries (all classes) staged in shared memory, 16 / gran per 16 bytes of K; 0: read in global memory
-    int32_t gran;               // bytes per gather copy: 16, 8 or 4
+    int32_t tab_entries;        // gather table entries (all classes) staged in shared memory, kBK / unit per k-block; 0: read in global memory
+    int32_t unit, unit_log2;    // bytes of the reduction per table entry: the largest of 16, 8 and 4 that divides the channels
+    int32_t gran;               // bytes per gather copy: unit, or less where the input pointer is not a multiple of it (1: byte by byte)
     int32_t cols_all;           // 1: the constants of every column are staged once
     int32_t need_asum, zw_eff, a_signed, act_min, act_max, out_zp, mode, sat_plain;
     uint32_t idesc;

@@ -1177,7 +1177,8 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     GcParams &p = gc->prm;
     p.n_classes = nc;
     p.N = N;
-    p.gran = (cin & 15) == 0 ? 16 : ((cin & 7) == 0 ? 8 : 4);
+    p.unit_log2 = (cin & 15) == 0 ? 4 : ((cin & 7) == 0 ? 3 : 2);
+    p.unit = 1 << p.unit_log2;
     p.h = g.h; p.w = g.w; p.cin = cin; p.sy = sy; p.sx = sx;
     p.out_sn = out_sn; p.out_sy = out_sy; p.out_sx = out_sx;
     p.zw_eff = g.w_signed ? g.w_zp : g.w_zp - 128;
@@ -1204,12 +1205,12 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         c.div_ow = FastDiv::make(static_cast<uint32_t>(d.ow));
         c.div_img = FastDiv::make(static_cast<uint32_t>(d.oh) * static_cast<uint32_t>(d.ow));
         c.out_base = d.out_base;
-        c.tab0 = kb_total * (kBK / p.gran);
+        c.tab0 = kb_total * (kBK / p.unit);
         tiles_m += c.tiles_m;
         kb_total += c.k_blocks;
         k_pad = std::max(k_pad, c.k_blocks * kBK);
     }
-    const int32_t tab_total = kb_total * (kBK / p.gran);
+    const int32_t tab_total = kb_total * (kBK / p.unit);
     p.tab_entries = tab_total <= 3072 ? tab_total : 0;      // 24 KB of gather table
     // N tiling: as few tiles as possible (every N tile gathers the A tile again), but split while SMs would idle.
     int32_t tiles_n = (N + max_data - 1) / max_data;
@@ -1234,7 +1235,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     // reductions of one or two k-blocks, whose time is the epilogue's.
     {
         const int64_t single = (p.n_units + sms - 1) / sms, pairs = (p.n_units + 2 * sms - 1) / (2 * sms);
-        const bool alone = p.n_units > sms && p.gran == 16 && kb_total > 2 * nc && single * 256 * 100 < pairs * (125 * 256 + 95 * p.bn_rows);
+        const bool alone = p.n_units > sms && p.unit == 16 && kb_total > 2 * nc && single * 256 * 100 < pairs * (125 * 256 + 95 * p.bn_rows);
         gc->per_sm = ctx->has_opt("gc_per_sm") ? (ctx->opt("gc_per_sm") == 1 ? 1 : 2) : (alone ? 1 : 2);
     }
     p.n_acc = gc->per_sm == 1 || 2 * p.bn_rows <= kMaxBN ? 2 : 1;      // half of the 512 columns per CTA, or all of them
@@ -1270,12 +1271,12 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         const GcClassDesc &d = classes[i];
         const int32_t K = d.kh * d.kw * cin;
         gc->gather_bytes = std::max(gc->gather_bytes, static_cast<size_t>(p.cls[i].M) * static_cast<size_t>((K + 15) & ~15));
-        for (int32_t k = 0; k < K; k += p.gran) {
+        for (int32_t k = 0; k < K; k += p.unit) {
             const int32_t tap = k / cin, c = k - tap * cin, ky = tap / d.kw, kx = tap - ky * d.kw;
             const int32_t dy = ky * d.dy, dx = kx * d.dx;
             const int64_t off = (static_cast<int64_t>(dy) * g.w + dx) * cin + c;
             if (off > INT32_MAX || off < INT32_MIN) return ENN_B200_INVALID_PARAMS;
-            tab[static_cast<size_t>(p.cls[i].tab0 + k / p.gran)] = make_int2(static_cast<int>(off), (dy << 16) | (dx & 0xffff));
+            tab[static_cast<size_t>(p.cls[i].tab0 + k / p.unit)] = make_int2(static_cast<int>(off), (dy << 16) | (dx & 0xffff));
         }
         for (int32_t n = 0; n < N; ++n) {
             int8_t *dst = wb.data() + ((static_cast<size_t>(i) * tiles_n + n / p.bn_data) * p.bn_rows + tile_row(n % p.bn_data, p.bn_data)) * k_pad;
@@ -1797,18 +1798,6 @@ void tc_set_residual(enn_b200_op *op, const void *res) {
 namespace {
 int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) {
     enn_b200_context *ctx = op->ctx;
-    if ((reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(plan->gcs[0]->prm.gran - 1)) != 0) {
-        // sub-buffers at odd offsets: the general kernels take any alignment
-        if (plan->fused_add) {
-            ctx->last_error = "fused convolution + add needs 16-byte aligned pointers";
-            return ENN_B200_INVALID_PARAMS;
-        }
-        const cudaError_t e = op->kind == OP_DECONV ? launch_deconv_direct(op->g, op->rq, in, op->w_direct, out, ctx->stream)
-                                                    : launch_conv_direct(op->g, op->rq, in, op->w_direct, out, ctx->stream);
-        if (e == cudaSuccess) return ENN_B200_SUCCESS;
-        ctx->last_error = std::string("kernel launch: ") + cudaGetErrorString(e);
-        return ENN_B200_CUDA_FAILURE;
-    }
     if (plan->fused_add) {
         if (!plan->residual || ((reinterpret_cast<uintptr_t>(plan->residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) {
             ctx->last_error = "fused convolution + add needs the second addend and 16-byte aligned pointers";
@@ -1823,6 +1812,9 @@ int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) 
         p.out = static_cast<uint8_t *>(out);
         p.add_res = plan->fused_add ? plan->residual : nullptr;
         p.test_starve = starve ? 1 : 0;
+        // sub-buffers at any offset: the widest copies that the pointer allows
+        p.gran = p.unit;
+        while (p.gran > 1 && (reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(p.gran - 1)) != 0) p.gran = p.gran > 4 ? p.gran / 2 : 1;
         const cudaError_t e = gconv_launch(*gc, ctx->stream);
         if (e != cudaSuccess) {
             ctx->last_error = std::string("gconv_kernel launch: ") + cudaGetErrorString(e);

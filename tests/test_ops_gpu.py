@@ -1279,7 +1279,7 @@ def test_gather_convolution(enn, orc, ctx, name):
     try:
         assert op.info.impl == enn.IMPL_TCGEN05 and op.info.kernel_launches == 1
         _check(op, y_ref, x)
-        buf = ctx.malloc(x.nbytes + 32)              # a sub-buffer at an odd offset: the general kernel takes it
+        buf = ctx.malloc(x.nbytes + 32)              # a sub-buffer at an odd offset
         out = ctx.malloc(y_ref.size)
         pin = type(buf)(buf.value + 1)
         ctx.upload(pin, x)
@@ -1295,6 +1295,33 @@ def test_gather_convolution(enn, orc, ctx, name):
         op.clear_error()
         _check(op, y_ref, x)
     finally:
+        op.release()
+
+
+@pytest.mark.parametrize("name", ["g16_resident_tail_k", "g16_staged_wide", "g8_k_tail", "g4_5x5_odd_n", "deconv_g8_four_classes", "deconv_g16_staged", "g16_table_in_global"])
+def test_gather_convolution_of_misaligned_input(enn, orc, ctx, name):
+    """Input pointers that are no multiple of the copies' size run the same kernel with narrower copies."""
+    kind, kw = GCONV_CASES[name]
+    mk, ref, case = (enn.conv2d, orc.conv2d, cases.conv_case) if kind == "conv" else (enn.deconv, orc.deconv, cases.deconv_case)
+    d, x, w, b, sc = case(seed=_seed("gconv_off_" + name), **kw)
+    y_ref = ref(d, x, w, b, sc)
+    op = mk(ctx, d, w, b, sc)
+    buf, out = ctx.malloc(x.nbytes + 32), ctx.malloc(y_ref.size)
+    try:
+        for off in (8, 4, 2, 1, 13):
+            pin = type(buf)(buf.value + off)
+            ctx.upload(pin, x)
+            op.execute(pin, out)
+            assert np.array_equal(ctx.download(out, (y_ref.size,), y_ref.dtype), y_ref.reshape(-1))
+            op.test_starve_next()                    # seen by the tensor-core kernel only: this pointer does not leave it
+            op.execute(pin, out)
+            ctx.sync()
+            with pytest.raises(enn.EnnError):
+                op.execute(pin, out)
+            op.clear_error()
+    finally:
+        ctx.free(buf)
+        ctx.free(out)
         op.release()
 
 
