@@ -137,7 +137,7 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
     const uint32_t rt = base + L.rows + static_cast<uint32_t>(t >> 5) * 512u, rt_lane = rt + static_cast<uint32_t>(lane / kPerRow) * 16;
     const int2 *const tab0 = (p.tab_entries ? reinterpret_cast<const int2 *>(sp + L.tab) : p.tab) + first;
     uint32_t stage = 0, phase = 0;
-    bool ok = !starve;
+    bool ok = !starve, waited = false;
     UnitWalk u;
     for (u.start(static_cast<int>(blockIdx.x)); ok && u.locate(p); u.unit += gridDim.x) {
         const GcClass &c = p.cls[u.c];
@@ -157,6 +157,10 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
             asm volatile("st.shared.b64 [%0], %1;\n\tst.shared.v2.b32 [%0 + 8], {%2, %3};" ::"r"(rt + lane * 16), "l"(row), "r"(iy), "r"(ix) : "memory");
         }
         __syncwarp();
+        if (!waited) {
+            pdl_wait();
+            waited = true;
+        }
         const uint8_t *rrow[G == 16 ? kPasses : 1];
         int riy[G == 16 ? kPasses : 1], rix[G == 16 ? kPasses : 1];
         if (G == 16) {
@@ -287,8 +291,12 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
                     tma_load_2d(base + static_cast<uint32_t>(p.cls[c].b_tile0 + tn * p.cls[c].k_blocks + kb) * p.b_bytes, &map_b, bres_bar, kb * kBK,
                                 (c * p.tiles_n + tn) * p.bn_rows);
     }
-    pdl_wait();
-    pdl_trigger();
+    // The gather warps wait for the kernel before once they have worked out the rows of their first unit (1x56x56x64 -> 64 4.5 -> 4.1 us,
+    // 16x28x28x72 -> 200 pointwise 6.15 -> 5.6).
+    if (warp < kEpiWarpsGc || warp >= kMmaWarp) {
+        pdl_wait();
+        pdl_trigger();
+    }
 
     const uint32_t stage_bytes = kBM * kBK + (p.b_res ? 0u : static_cast<uint32_t>(p.b_bytes));
     if (warp >= kEpiWarpsGc && warp < kMmaWarp) {
