@@ -13,6 +13,7 @@
 #include <new>
 
 #include "internal.h"
+#include "per_device.h"
 #include "requant.h"
 
 namespace enn_b200 {
@@ -684,6 +685,32 @@ struct DwRingPlan {
     void *zrow_dev = nullptr;          // row of input zero points
 };
 
+namespace {
+template <int ST, bool WS, bool AS, bool BIG>
+cudaError_t set_ring_attr() {
+    cudaError_t e = cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 0, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 1, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 2, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+    return e;
+}
+template <int ST, bool WS, bool AS>
+cudaError_t set_ring_attrs() {
+    const cudaError_t e = set_ring_attr<ST, WS, AS, false>();
+    return e == cudaSuccess ? set_ring_attr<ST, WS, AS, true>() : e;
+}
+cudaError_t ring_init(int device) {
+    static PerDeviceInit once;
+    return once.run(device, [] {
+        cudaError_t e = cudaSuccess;
+        for (const cudaError_t each : {set_ring_attrs<1, true, true>(), set_ring_attrs<1, true, false>(), set_ring_attrs<1, false, true>(),
+                                       set_ring_attrs<1, false, false>(), set_ring_attrs<2, true, true>(), set_ring_attrs<2, true, false>(),
+                                       set_ring_attrs<2, false, true>(), set_ring_attrs<2, false, false>()})
+            if (each != cudaSuccess) e = each;
+        return e;
+    });
+}
+}  // namespace
+
 // Chooses tile width, ring depth and grid; returns false when the geometry is outside the kernel's domain.
 bool dw_ring_plan(enn_b200_op *op) {
     const ConvGeom &g = op->g;
@@ -698,6 +725,10 @@ bool dw_ring_plan(enn_b200_op *op) {
     const int ns = (strips + tx_n - 1) / tx_n;
     // every x tile must hold at least one pixel of the image: a tile without one has no copies and nothing to wait for
     if ((tx_n - 1) * ns * 4 * s - g.pl >= g.w || (4 * ns - 1) * s + 3 <= g.pl) return false;
+    if (ring_init(ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     DwRingPlan *pl = new (std::nothrow) DwRingPlan();
     if (!pl) return false;
     DwRingParams &p = pl->prm;
@@ -783,20 +814,6 @@ cudaError_t dw_ring_launch(enn_b200_op *op, const void *in, void *out) {
     cudaStream_t s = op->ctx->stream;
     const bool asum = g.w_zp != 0;
     const int rq = !op->dw_relu ? 0 : ((g.act_min == 0 && g.act_max >= 255) ? 2 : 1);
-    static bool attr_set = false;
-#define ENN_DWR_ATTR(ST, WS, AS) \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024); \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024); \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024); \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024); \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024); \
-    cudaFuncSetAttribute(dw3x3_ring_kernel<ST, WS, AS, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024)
-    if (!attr_set) {
-        ENN_DWR_ATTR(1, true, true); ENN_DWR_ATTR(1, true, false); ENN_DWR_ATTR(1, false, true); ENN_DWR_ATTR(1, false, false);
-        ENN_DWR_ATTR(2, true, true); ENN_DWR_ATTR(2, true, false); ENN_DWR_ATTR(2, false, true); ENN_DWR_ATTR(2, false, false);
-        attr_set = true;
-    }
-#undef ENN_DWR_ATTR
     const bool big = pl->threads > kDwRingThreads;
 #define ENN_DWR(ST, WS, AS, RQ)                                                                                                            \
     (big ? launch_pdl(dw3x3_ring_kernel<ST, WS, AS, RQ, true>, dim3(pl->grid), dim3(pl->threads), pl->smem, s, pl->prm, c, w, i, o) \

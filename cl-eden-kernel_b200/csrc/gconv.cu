@@ -16,6 +16,7 @@
 //
 // Every wait is bounded (tc_common.cuh): on expiry an error code reaches the host and all roles fall through to the exit.
 #include "gconv.cuh"
+#include "per_device.h"
 
 #include <type_traits>
 
@@ -457,12 +458,12 @@ uint32_t gconv_smem_bytes(const GcParams &p, uint32_t b_res_bytes) {
     return gc_smem(p, b_res_bytes, cols).total + 1024;       // 1024: alignment of the tiles
 }
 
-cudaError_t gconv_init() {
-    static cudaError_t once = [] {
-        cudaError_t e = set_attrs<false>();
+cudaError_t gconv_init(int device) {
+    static PerDeviceInit once;
+    return once.run(device, [] {
+        const cudaError_t e = set_attrs<false>();
         return e == cudaSuccess ? set_attrs<true>() : e;
-    }();
-    return once;
+    });
 }
 
 cudaError_t gconv_launch(const GcPlan &plan, cudaStream_t s) { return plan.prm.need_asum ? launch_mode<true>(plan, s) : launch_mode<false>(plan, s); }

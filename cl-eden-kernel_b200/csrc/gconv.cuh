@@ -93,6 +93,6 @@ constexpr int kGcMaxStages = 8;
 
 uint32_t gconv_smem_bytes(const GcParams &p, uint32_t b_res_bytes);
 cudaError_t gconv_launch(const GcPlan &plan, cudaStream_t stream);
-cudaError_t gconv_init();
+cudaError_t gconv_init(int device);      // with `device` current
 
 }  // namespace enn_b200

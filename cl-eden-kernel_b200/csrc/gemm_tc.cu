@@ -32,6 +32,7 @@
 #include "tc_common.cuh"
 #include "tc_host.h"
 #include "gconv.cuh"
+#include "per_device.h"
 
 namespace enn_b200 {
 
@@ -1309,7 +1310,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         (e = cudaMalloc(&gc->tab_dev, tab.size() * sizeof(int2))) != cudaSuccess ||
         (e = cudaMemcpy(gc->w_dev, wb.data(), wb.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(gc->cols_dev, cols.data(), cols.size() * sizeof(ColParam), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(gc->tab_dev, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice)) != cudaSuccess || (e = gconv_init()) != cudaSuccess) {
+        (e = cudaMemcpy(gc->tab_dev, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice)) != cudaSuccess || (e = gconv_init(ctx->device)) != cudaSuccess) {
         ctx->last_error = std::string("gather convolution plan: ") + cudaGetErrorString(e);
         return ENN_B200_CUDA_FAILURE;
     }
@@ -1429,10 +1430,28 @@ void launch_tc_gemm(const TcGemm &gm, const CUtensorMap &map_a, const TcParams &
     else launch_tc_gemm_mode<false>(gm, map_a, p, stream);
 }
 
-template <bool ASUM, int MODE>
-void set_tc_gemm_smem_attr() {
-    cudaFuncSetAttribute(tc_gemm_kernel<ASUM, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(tc_gemm_kernel<ASUM, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+template <bool ASUM, int MODE, bool TWO, bool FADD = false>
+cudaError_t set_tc_gemm_attr() {
+    return cudaFuncSetAttribute(tc_gemm_kernel<ASUM, MODE, TWO, FADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+template <bool ASUM>
+cudaError_t set_tc_gemm_attrs() {
+    cudaError_t e = cudaSuccess;
+    for (const cudaError_t each : {set_tc_gemm_attr<ASUM, kModeNudge, false>(), set_tc_gemm_attr<ASUM, kModeNudge, true>(),
+                                   set_tc_gemm_attr<ASUM, kModeGeneral, false>(), set_tc_gemm_attr<ASUM, kModeGeneral, true>(),
+                                   set_tc_gemm_attr<ASUM, kModeReluHi, false>(), set_tc_gemm_attr<ASUM, kModeReluHi, true>(),
+                                   set_tc_gemm_attr<ASUM, kModeReluTwo, false>(), set_tc_gemm_attr<ASUM, kModeReluTwo, true>(),
+                                   set_tc_gemm_attr<ASUM, kModeReluSat, false>(), set_tc_gemm_attr<ASUM, kModeReluSat, true>(),
+                                   set_tc_gemm_attr<ASUM, kModeNudge, false, true>(), set_tc_gemm_attr<ASUM, kModeGeneral, false, true>()})
+        if (each != cudaSuccess) e = each;
+    return e;
+}
+cudaError_t tc_gemm_init(int device) {
+    static PerDeviceInit once;
+    return once.run(device, [] {
+        const cudaError_t e = set_tc_gemm_attrs<false>();
+        return e == cudaSuccess ? set_tc_gemm_attrs<true>() : e;
+    });
 }
 
 }  // namespace
@@ -1735,23 +1754,9 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         }
     }
     op->info.kernel_launches = launches;
-    static bool attr_set = false;
-    if (!attr_set) {
-        set_tc_gemm_smem_attr<false, kModeNudge>();
-        set_tc_gemm_smem_attr<false, kModeGeneral>();
-        set_tc_gemm_smem_attr<false, kModeReluHi>();
-        set_tc_gemm_smem_attr<false, kModeReluTwo>();
-        set_tc_gemm_smem_attr<false, kModeReluSat>();
-        set_tc_gemm_smem_attr<true, kModeNudge>();
-        set_tc_gemm_smem_attr<true, kModeGeneral>();
-        set_tc_gemm_smem_attr<true, kModeReluHi>();
-        set_tc_gemm_smem_attr<true, kModeReluTwo>();
-        set_tc_gemm_smem_attr<true, kModeReluSat>();
-        cudaFuncSetAttribute(tc_gemm_kernel<false, kModeNudge, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(tc_gemm_kernel<false, kModeGeneral, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(tc_gemm_kernel<true, kModeNudge, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(tc_gemm_kernel<true, kModeGeneral, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr_set = true;
+    if ((e = tc_gemm_init(ctx->device)) != cudaSuccess) {
+        ctx->last_error = std::string("tensor-core plan: ") + cudaGetErrorString(e);
+        return bail(ENN_B200_CUDA_FAILURE);
     }
     op->tc = plan;
     return ENN_B200_SUCCESS;
