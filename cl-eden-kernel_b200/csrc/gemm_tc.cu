@@ -1237,7 +1237,9 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     {
         const int64_t single = (p.n_units + sms - 1) / sms, pairs = (p.n_units + 2 * sms - 1) / (2 * sms);
         const bool alone = p.n_units > sms && p.unit == 16 && kb_total > 2 * nc && single * 256 * 100 < pairs * (125 * 256 + 95 * p.bn_rows);
-        gc->per_sm = ctx->has_opt("gc_per_sm") ? (ctx->opt("gc_per_sm") == 1 ? 1 : 2) : (alone ? 1 : 2);
+        // A share of the SMs (option grid_cap) is that many CTAs, of which each may have an SM for itself.
+        if (sms < ctx->sm_count) gc->per_sm = 1;
+        else gc->per_sm = ctx->has_opt("gc_per_sm") ? (ctx->opt("gc_per_sm") == 1 ? 1 : 2) : (alone ? 1 : 2);
     }
     p.n_acc = gc->per_sm == 1 || 2 * p.bn_rows <= kMaxBN ? 2 : 1;      // half of the 512 columns per CTA, or all of them
     p.tmem_cols = 32;

@@ -1014,6 +1014,49 @@ def test_grid_cap_keeps_results(enn, orc, name, cap):
         c.close()
 
 
+def _captured_grids(ctx, launch):
+    """CTAs of every kernel that `launch` enqueues on the context's stream, read from a stream capture (nothing runs)."""
+    from cuda.bindings import driver as drv
+
+    def ok(r):
+        assert r[0] == drv.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    stream = drv.CUstream(ctx.stream)
+    ok(drv.cuStreamBeginCapture(stream, drv.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_THREAD_LOCAL))
+    try:
+        launch()
+    finally:
+        graph = ok(drv.cuStreamEndCapture(stream))
+    try:
+        count = ok(drv.cuGraphGetNodes(graph))[1]
+        nodes = ok(drv.cuGraphGetNodes(graph, count))[0]
+        prm = [ok(drv.cuGraphKernelNodeGetParams(n)) for n in nodes if ok(drv.cuGraphNodeGetType(n)) == drv.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL]
+        return [p.gridDimX * p.gridDimY * p.gridDimZ for p in prm]
+    finally:
+        drv.cuGraphDestroy(graph)
+
+
+@pytest.mark.parametrize("cap", [1, 7, 37])
+@pytest.mark.parametrize("name", ["conv3x3_tapbox", "deconv", "conv1x1_wide_n"])
+def test_grid_cap_bounds_the_tensor_core_grids(enn, name, cap):
+    """Option grid_cap = G: at most G CTAs per tensor-core launch."""
+    kind, (d, x, w, b, s) = GRID_CAP_CASES[name]()
+    d.n = 40                                  # more units than any of the shares
+    c = enn.Context(0)
+    try:
+        c.set_option("grid_cap", cap)
+        op = (enn.deconv if kind == "deconv" else enn.conv2d)(c, d, w, b, s)
+        a, o = c.malloc(op.info.in_bytes), c.malloc(op.info.out_bytes)
+        grids = _captured_grids(c, lambda: op.execute(a, o))
+        assert len(grids) == op.info.kernel_launches and max(grids) <= cap
+        c.free(a)
+        c.free(o)
+        op.release()
+    finally:
+        c.close()
+
+
 def test_oplist_group_splits_one_batch(enn, orc):
     """enn_b200_group_*: one host batch in, one host buffer out, over three operator lists with slices of 3 + 2 + 1
     images (their own contexts; on a one-GPU machine all on device 0): blocking and pipelined calls equal the oracle on
