@@ -76,6 +76,7 @@ struct GcPlan {
     CUtensorMap map_b{};
     void *w_dev = nullptr, *cols_dev = nullptr, *tab_dev = nullptr;
     size_t smem_bytes = 0;
+    uint32_t b_res_bytes = 0;   // resident weights
     int grid = 0;
     int per_sm = 2;             // CTAs the shared memory is laid out for
     size_t gather_bytes = 0;    // what the matrix would take if it were materialised (limit of the allocation-free call)

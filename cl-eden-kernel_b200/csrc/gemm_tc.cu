@@ -1260,6 +1260,7 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     // staged tile by tile, and at last the table stays in global memory (what is left, 96 + 4 + 2 KB and the barriers, always fits).
     if (gconv_smem_bytes(p, b_res_bytes) > limit) p.cols_all = 0;
     if (gconv_smem_bytes(p, b_res_bytes) > limit) p.tab_entries = 0;
+    gc->b_res_bytes = b_res_bytes;
     gc->smem_bytes = std::max<size_t>(gconv_smem_bytes(p, b_res_bytes), gc->per_sm == 1 ? kGcSmemLimit + 2048 : 0);
     gc->grid = std::min(p.n_units, gc->per_sm * sms);
 
@@ -1773,10 +1774,12 @@ int32_t tc_fuse_add(enn_b200_op *op, const AddParams &add, bool conv_is_second) 
         GcParams &p = gc.prm;
         if (op->kind != OP_CONV || (p.mode != kModeNudge && p.mode != kModeGeneral) || (p.N & 15) != 0 || !add.lut || add.is_signed != p.a_signed)
             return ENN_B200_INVALID_PARAMS;
-        if (gc.smem_bytes + 2048 > kGcSmemLimit) return ENN_B200_INVALID_PARAMS;
-        gc.smem_bytes += 2048;
         p.add = add;
         p.add_on = 1;
+        // Room for the tables: a stage less where they do not fit, at last one CTA per SM.
+        const size_t limit = gc.per_sm == 1 ? kGcSmemAlone : kGcSmemLimit;
+        while (p.stages > 2 && gconv_smem_bytes(p, gc.b_res_bytes) > limit) --p.stages;
+        gc.smem_bytes = std::max<size_t>(gconv_smem_bytes(p, gc.b_res_bytes), gc.per_sm == 1 ? gc.smem_bytes : 0);
         p.add_swap = conv_is_second ? 1 : 0;
         plan->fused_add = true;
         return ENN_B200_SUCCESS;

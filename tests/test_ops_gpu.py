@@ -749,6 +749,10 @@ FUSED_ADD_CASES = {
     "project_7x7_960_to_160": (dict(n=9, h=7, w=7, cin=960, cout=160, k=1, per_channel=True, out_scale=0.25, act=0, out_zp=130), False),
     "u8_weights_partial_tile": (dict(n=1, h=19, w=21, cin=64, cout=48, k=1, w_zp=131, out_scale=0.06, act=0, out_zp=119), False),
     "implicit_3x3": (dict(n=2, h=12, w=13, cin=32, cout=32, k=3, per_channel=True, out_scale=0.5, act=0, out_zp=125), True),
+    # plans that leave less than the add's 2 KB of shared memory: two CTAs per SM (three and four stages), one per SM
+    "gather_full": (dict(n=1, h=14, w=14, cin=64, cout=96, k=3, per_channel=True, out_scale=0.5, act=0, out_zp=125), False),
+    "gather_nearly_full": (dict(n=1, h=14, w=14, cin=144, cout=32, k=3, per_channel=True, out_scale=0.5, act=0, out_zp=125), True),
+    "gather_alone": (dict(n=1, h=139, w=140, cin=64, cout=256, k=3, per_channel=True, out_scale=0.5, act=0, out_zp=125), False),
 }
 
 
