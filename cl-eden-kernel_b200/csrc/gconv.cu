@@ -420,19 +420,17 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
 }
 
 template <bool ASUM, int MODE, bool FADD = false>
-cudaError_t launch_one(const GcPlan &plan, cudaStream_t s) {
-    return launch_pdl(gconv_kernel<ASUM, MODE, FADD>,
-                      dim3(static_cast<unsigned>(plan.grid)), dim3(kGcThreads), plan.smem_bytes, s, plan.map_b, plan.prm);
+cudaError_t launch_one(const GcPlan &plan, const GcParams &p, cudaStream_t s) {
+    return launch_pdl(gconv_kernel<ASUM, MODE, FADD>, dim3(static_cast<unsigned>(plan.grid)), dim3(kGcThreads), plan.smem_bytes, s, plan.map_b, p);
 }
 template <bool ASUM>
-cudaError_t launch_mode(const GcPlan &plan, cudaStream_t s) {
-    const GcParams &p = plan.prm;
-    if (p.add_on) return p.mode == kModeNudge ? launch_one<ASUM, kModeNudge, true>(plan, s) : launch_one<ASUM, kModeGeneral, true>(plan, s);
+cudaError_t launch_mode(const GcPlan &plan, const GcParams &p, cudaStream_t s) {
+    if (p.add_on) return p.mode == kModeNudge ? launch_one<ASUM, kModeNudge, true>(plan, p, s) : launch_one<ASUM, kModeGeneral, true>(plan, p, s);
     switch (p.mode) {
-        case kModeNudge: return launch_one<ASUM, kModeNudge>(plan, s);
-        case kModeGeneral: return launch_one<ASUM, kModeGeneral>(plan, s);
-        case kModeReluHi: return p.sat_plain ? launch_one<ASUM, kModeReluSat>(plan, s) : launch_one<ASUM, kModeReluHi>(plan, s);
-        default: return launch_one<ASUM, kModeReluTwo>(plan, s);
+        case kModeNudge: return launch_one<ASUM, kModeNudge>(plan, p, s);
+        case kModeGeneral: return launch_one<ASUM, kModeGeneral>(plan, p, s);
+        case kModeReluHi: return p.sat_plain ? launch_one<ASUM, kModeReluSat>(plan, p, s) : launch_one<ASUM, kModeReluHi>(plan, p, s);
+        default: return launch_one<ASUM, kModeReluTwo>(plan, p, s);
     }
 }
 template <bool ASUM, int MODE, bool FADD = false>
@@ -466,6 +464,6 @@ cudaError_t gconv_init(int device) {
     });
 }
 
-cudaError_t gconv_launch(const GcPlan &plan, cudaStream_t s) { return plan.prm.need_asum ? launch_mode<true>(plan, s) : launch_mode<false>(plan, s); }
+cudaError_t gconv_launch(const GcPlan &plan, const GcParams &p, cudaStream_t s) { return p.need_asum ? launch_mode<true>(plan, p, s) : launch_mode<false>(plan, p, s); }
 
 }  // namespace enn_b200

@@ -93,7 +93,7 @@ constexpr uint32_t kGcSmemLimit = 113 * 1024, kGcSmemAlone = 227 * 1024;      //
 constexpr int kGcMaxStages = 8;
 
 uint32_t gconv_smem_bytes(const GcParams &p, uint32_t b_res_bytes);
-cudaError_t gconv_launch(const GcPlan &plan, cudaStream_t stream);
+cudaError_t gconv_launch(const GcPlan &plan, const GcParams &prm, cudaStream_t stream);      // prm: the plan's, completed by the call
 cudaError_t gconv_init(int device);      // with `device` current
 
 }  // namespace enn_b200

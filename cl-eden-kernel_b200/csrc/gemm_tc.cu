@@ -1806,26 +1806,23 @@ void tc_set_residual(enn_b200_op *op, const void *res) {
 }
 
 namespace {
-int32_t gconv_execute(enn_b200_op *op, TcPlan *plan, const void *in, void *out) {
+// Launches a gather convolution with parameters of this call only; the plan stays as it is.  `residual`: other addend of a fused add.
+int32_t gconv_execute(const enn_b200_op *op, const TcPlan *plan, const void *in, void *out, const uint8_t *residual, bool starve) {
     enn_b200_context *ctx = op->ctx;
-    if (plan->fused_add) {
-        if (!plan->residual || ((reinterpret_cast<uintptr_t>(plan->residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) {
-            ctx->last_error = "fused convolution + add needs the second addend and 16-byte aligned pointers";
-            return ENN_B200_INVALID_PARAMS;
-        }
+    if (plan->fused_add && (!residual || ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0)) {
+        ctx->last_error = "fused convolution + add needs the second addend, and it and the output 16-byte aligned";
+        return ENN_B200_INVALID_PARAMS;
     }
-    const bool starve = plan->starve_next;
-    plan->starve_next = false;
     for (auto &gc : plan->gcs) {
-        GcParams &p = gc->prm;
+        GcParams p = gc->prm;
         p.in = static_cast<const uint8_t *>(in);
         p.out = static_cast<uint8_t *>(out);
-        p.add_res = plan->fused_add ? plan->residual : nullptr;
+        p.add_res = residual;
         p.test_starve = starve ? 1 : 0;
         // sub-buffers at any offset: the widest copies that the pointer allows
         p.gran = p.unit;
         while (p.gran > 1 && (reinterpret_cast<uintptr_t>(in) & static_cast<uintptr_t>(p.gran - 1)) != 0) p.gran = p.gran > 4 ? p.gran / 2 : 1;
-        const cudaError_t e = gconv_launch(*gc, ctx->stream);
+        const cudaError_t e = gconv_launch(*gc, p, ctx->stream);
         if (e != cudaSuccess) {
             ctx->last_error = std::string("gconv_kernel launch: ") + cudaGetErrorString(e);
             return ENN_B200_CUDA_FAILURE;
@@ -1845,9 +1842,9 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = buf;
         return ENN_B200_CUDA_FAILURE;
     }
-    if (!plan->gcs.empty()) return gconv_execute(op, plan, in, out);
     const bool starve = plan->starve_next;
     plan->starve_next = false;
+    if (!plan->gcs.empty()) return gconv_execute(op, plan, in, out, plan->residual, starve);
     for (auto &gm : plan->gemms) {
         TcParams &p = gm.prm;
         if (p.M == 0) continue;
@@ -1994,7 +1991,7 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
         return ENN_B200_INVALID_PARAMS;
     }
     if (!plan->gcs.empty()) {      // gathers into shared memory: no scratch array needed
-        if (*plan->err_host == 0) return gconv_execute(op, plan, in, out);
+        if (*plan->err_host == 0) return gconv_execute(op, plan, in, out, nullptr, false);
         ctx->last_error = "gather convolution gave up on a barrier wait earlier";
         return ENN_B200_CUDA_FAILURE;
     }

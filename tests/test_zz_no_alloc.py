@@ -76,3 +76,22 @@ def test_noalloc_rejects_what_it_cannot_hold(enn, ctx):
         ctx.free(a)
         ctx.free(o)
         op.release()
+
+
+def test_noalloc_leaves_the_launch_state_alone(enn, ctx):
+    """An armed self-test waits for the regular entry point: the allocation-free call in between is an ordinary one."""
+    for kw in (dict(n=1, h=9, w=9, cin=16, cout=16, k=3), dict(n=1, h=9, w=9, cin=6, cout=16, k=3)):      # gathered inside the kernel; into the array
+        d, x, w, b, sc = cases.conv_case(seed=23, **kw)
+        op = enn.conv2d(ctx, d, w, b, sc)
+        try:
+            want = op.run(x)
+            op.test_starve_next()
+            assert np.array_equal(_run_noalloc(enn, ctx, op, x), want)
+            op.run(x)                                    # this launch gives up
+            ctx.sync()
+            with pytest.raises(enn.EnnError):
+                op.run(x)
+            op.clear_error()
+            assert np.array_equal(op.run(x), want)
+        finally:
+            op.release()
