@@ -1836,6 +1836,8 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
     TcPlan *plan = static_cast<TcPlan *>(op->tc);
     enn_b200_context *ctx = op->ctx;
     if (!plan) return ENN_B200_FAILURE;
+    const uint8_t *residual = plan->residual;
+    plan->residual = nullptr;          // for this call only: the tensor may be gone by the next one
     if (*plan->err_host != 0) {
         char buf[96];
         std::snprintf(buf, sizeof(buf), "tensor-core kernel gave up on a barrier wait (code %d)", *plan->err_host);
@@ -1844,7 +1846,7 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
     }
     const bool starve = plan->starve_next;
     plan->starve_next = false;
-    if (!plan->gcs.empty()) return gconv_execute(op, plan, in, out, plan->residual, starve);
+    if (!plan->gcs.empty()) return gconv_execute(op, plan, in, out, residual, starve);
     for (auto &gm : plan->gemms) {
         TcParams &p = gm.prm;
         if (p.M == 0) continue;
@@ -1897,11 +1899,11 @@ int32_t tc_execute(enn_b200_op *op, const void *in, void *out) {
         }
         p.out = static_cast<uint8_t *>(out);
         if (plan->fused_add) {
-            if (!plan->residual || ((reinterpret_cast<uintptr_t>(plan->residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) {
+            if (!residual || ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(out)) & 15) != 0) {
                 ctx->last_error = "fused convolution + add needs the second addend and 16-byte aligned pointers";
                 return ENN_B200_INVALID_PARAMS;
             }
-            p.add_res = plan->residual;
+            p.add_res = residual;
         }
         p.test_starve = starve ? 1 : 0;
 #ifdef ENN_B200_DEV

@@ -788,6 +788,28 @@ def test_conv_with_fused_add(enn, orc, ctx, name):
         op.release()
 
 
+@pytest.mark.parametrize("name", ["project_7x7_960_to_160", "implicit_3x3"])
+def test_fused_addend_belongs_to_its_call(enn, ctx, name):
+    """A later call without the second addend is refused: the pointer of the one before is not kept."""
+    kw, conv_second = FUSED_ADD_CASES[name]
+    d, x, w, b, sc = cases.conv_case(seed=5, **kw)
+    op = enn.conv2d(ctx, d, w, b, sc)
+    addop = enn.add(ctx, enn.AddDesc(count=op.info.out_bytes, activation=0, act_dtype=enn.U8, in0_scale=0.031, in0_zp=120, in1_scale=0.047,
+                                     in1_zp=131, out_scale=0.06, out_zp=126))
+    size = op.info.out_bytes
+    op.fuse_add(addop, conv_second)
+    xd, rd, od = ctx.to_device(x), ctx.to_device(np.zeros(size, np.uint8)), ctx.malloc(size)
+    try:
+        op.execute2(xd, rd, od)
+        with pytest.raises(enn.EnnError):
+            op.execute(xd, od)
+        ctx.sync()
+    finally:
+        for p_ in (xd, rd, od):
+            ctx.free(p_)
+        op.release()
+
+
 def test_fused_add_refusals(enn, ctx):
     d, x, w, b, sc = cases.conv_case(seed=5, n=2, h=14, w=14, cin=32, cout=48, k=1, per_channel=True, out_scale=0.0235, out_zp=0)   # ReLU6: merged epilogue
     op = enn.conv2d(ctx, d, w, b, sc)
