@@ -491,11 +491,10 @@ dw3x3_ring_kernel(const DwRingParams p, const DwChan *__restrict__ chan, const u
                 }
                 u += cnt;
             }
-            if (!ok) {      // copies still in flight get a bounded chance to land before the shared memory is given back
-                for (int s2 = 0; s2 < p.nr; ++s2)
-                    for (uint32_t i = 0; i < (1u << 16); ++i)
-                        if (dw_mbar_try(full0 + 8 * s2, 0) || dw_mbar_try(full0 + 8 * s2, 1)) break;
-            }
+            if (!ok)        // copies in flight get a bounded chance to land before the shared memory is given back; a slot's last fill was in
+                for (uint32_t s2 = 0; s2 < static_cast<uint32_t>(p.nr); ++s2)      // the ring's present round before `slot`, else in the one before
+                    for (uint32_t i = 0; i < (1u << 12); ++i)
+                        if (dw_mbar_try(full0 + 8 * s2, s2 < slot ? phase : phase ^ 1)) break;
         }
         return;
     }

@@ -319,10 +319,10 @@ __global__ void __launch_bounds__(kGcThreads, 2) gconv_kernel(const __grid_const
                     if (++stage == static_cast<uint32_t>(nst)) { stage = 0; phase ^= 1; }
                 }
             }
-            if (!ok)        // give copies already in flight a bounded chance to land before shared memory is released
-                for (int s = 0; s < nst; ++s)
-                    for (uint32_t i = 0; i < (1u << 16); ++i)
-                        if (mbar_try_wait(full0 + 8 * s, 0) || mbar_try_wait(full0 + 8 * s, 1)) break;
+            if (!ok) drain_stages(full0, nst, stage, phase);
+        } else if (p.b_res && lane == 0 && !starve) {
+            for (uint32_t i = 0; i < (1u << 12); ++i)        // the MMA role may have given up before they landed
+                if (mbar_try_wait(bres_bar, 0)) break;
         }
     } else if (warp == kMmaWarp) {
         if (lane == 0) {

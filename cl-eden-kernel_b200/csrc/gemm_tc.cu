@@ -313,11 +313,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     kb += nl;
                     while (kb >= p.k_blocks) { kb -= p.k_blocks; ++t; }
                 }
-                if (!ok) {
-                    for (int s2 = 0; s2 < nst; ++s2)
-                        for (uint32_t i = 0; i < (1u << 16); ++i)
-                            if (mbar_try_wait(full0 + 8 * s2, 0) || mbar_try_wait(full0 + 8 * s2, 1)) break;
-                }
+                if (!ok && rank == 0) drain_stages(full0, nst, stage, phase, lane, nl);      // a pair's copies report to rank 0
             }
         } else if (!starve && !TWO && !split && bres && (nst & 1) == 0 && !(ENN_DBG_MODE(p) & 9)) {
             // Resident weights (narrow pointwise layers): only A tiles are left to load, and the copy
@@ -361,11 +357,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     if (stage >= static_cast<uint32_t>(nst)) { stage -= nst; phase ^= 1; }
                     advance(2);
                 }
-                if (!ok) {
-                    for (int s2 = 0; s2 < nst; ++s2)
-                        for (uint32_t i = 0; i < (1u << 16); ++i)
-                            if (mbar_try_wait(full0 + 8 * s2, 0) || mbar_try_wait(full0 + 8 * s2, 1)) break;
-                }
+                if (!ok) drain_stages(full0, nst, stage, phase, lane, 2);
             }
         } else if (lane == 0 && !starve) {
             // WHICH: 0 = the A tiles, 1 = the B tiles, 2 = both (launches without the separate B producer warp)
@@ -421,12 +413,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
                 if (dbg && DO_A) ENN_DBG_PTR(p)[blockIdx.x * 8 + 0] = t_wait;
-                if (!ok) {
-                    // Give copies already in flight a bounded chance to land before shared memory is released.
-                    for (int s = 0; s < nst; ++s)
-                        for (uint32_t i = 0; i < (1u << 16); ++i)
-                            if (mbar_try_wait(full0 + 8 * s, 0) || mbar_try_wait(full0 + 8 * s, 1)) break;
-                }
+                if (!ok && rank == 0) drain_stages(full0, nst, stage, phase);      // a pair's copies report to rank 0
             };
             if (!split) produce(std::integral_constant<int, 2>{});
             else if (warp == 0) produce(std::integral_constant<int, 0>{});

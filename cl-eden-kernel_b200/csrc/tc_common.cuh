@@ -88,6 +88,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return false;
 }
 
+// A producer that gives up waits, with a limit, for its copies in flight before the shared memory is given back.  (stage, phase) is the
+// next fill: stages before it were last filled in the ring's present round, the others in the round before (never filled: nothing to
+// wait for).  Lanes that fill alternate stages pass theirs as first and step.
+__device__ __forceinline__ void drain_stages(uint32_t full0, uint32_t nst, uint32_t stage, uint32_t phase, uint32_t first = 0, uint32_t step = 1) {
+    for (uint32_t s = first; s < nst; s += step)
+        for (uint32_t i = 0; i < (1u << 12); ++i)
+            if (mbar_try_wait(full0 + 8 * s, s < stage ? phase : phase ^ 1)) break;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t c0, int32_t c1) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
