@@ -1,9 +1,10 @@
-// gconv_kernel: gather convolution on the tensor cores, one launch per operator.
+// gconv_kernel: gather convolution on the tensor cores, one launch per operator (transposed convolutions of stride 4 and more: one per
+// nine parity classes).
 //
-// Two CTAs per SM, each warp-specialised:
-//   warps 0..3  epilogue: tcgen05.ld, requantisation, stores (one accumulator row = one output pixel per thread)
+// Two CTAs per SM, or one (build_gconv says where), each warp-specialised:
+//   warps 0..3  epilogue: tcgen05.ld, requantisation, stores (quad form, tc_common.cuh: four rows of the same columns per thread)
 //   warps 4..7  gather: the A tile of a k-block (128 output pixels x 128 reduction bytes) is fetched from the NHWC tensor with
-//               16-, 8- or 4-byte asynchronous copies straight into the 128-byte-swizzled operand layout; positions outside
+//               16-byte asynchronous copies, or 8-, 4- or 1-byte loads, straight into the 128-byte-swizzled operand layout; positions outside
 //               the image are stored as the input zero point
 //   warp 8      TMEM allocation, MMA issue
 //   warp 9      TMA copies of the packed weights (once per CTA when they fit, else per k-block)

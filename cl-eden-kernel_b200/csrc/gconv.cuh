@@ -79,7 +79,7 @@ struct GcPlan {
     uint32_t b_res_bytes = 0;   // resident weights
     int grid = 0;
     int per_sm = 2;             // CTAs the shared memory is laid out for
-    size_t gather_bytes = 0;    // what the matrix would take if it were materialised (limit of the allocation-free call)
+    size_t gather_bytes = 0;    // what the gathered matrix would take: the allocation-free call's limit, which no kernel's choice moves
 };
 
 // Geometry of one class for the planner; row m = (image, oy, ox), column k = (ky * kw + kx) * cin + c, input pixel

@@ -5,8 +5,8 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0      TMA producer of the A tiles (one lane)
 //   warp 1      TMEM allocation, MMA issue (one lane)
-//   warps 2..13 epilogue: each thread owns one accumulator row (= one output pixel) and a share of its columns
-//   warp 14     TMA producer of the B tiles (one lane)
+//   warps 2..9  epilogue (quad form, tc_common.cuh): two warps per TMEM lane quarter share the groups of 32 columns
+//   warp 10     TMA producer of the B tiles (one lane; long K only)
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the MMAs of tile i+1.
 //
 // Value computed (ConvolutionKernels.cpp:956-1274 / :1317-1375): for output row m, column n
@@ -57,9 +57,9 @@ namespace {
 #define ENN_DBG_PTR(p) static_cast<long long *>(nullptr)
 #endif
 
-// Epilogue warps: 3 per TMEM lane quarter, splitting the 16-column chunks.  The epilogue is bound by dependent integer
-// latencies, not by warp count: 12 warps with 128 registers (room for the compiler to interleave the 8 outputs of a half
-// chunk) run the MobileNetV2 graph 6 % faster than 24 warps capped at 72 registers; 8 and 16 warps are 1 % behind.
+// Epilogue warps: two per TMEM lane quarter, which share the groups of 32 columns.  Eight were chosen on an epilogue of one row per
+// thread that took up to 168 registers (16 -> 96 expand layer 140 us with twelve warps of 128, 126 us with eight).  In quad form the
+// kernels without activation sums take 118 to 128, so twelve would fit again; not measured.
 constexpr int kEpiWarps = 8;
 constexpr int kColGroups = kEpiWarps / 4;
 constexpr int kGroupsPerWarp = kMaxBN / 32 / kColGroups;   // column groups one warp can own
@@ -1004,8 +1004,8 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
                    TcGemm *gm, bool want_resident = false) {
     TcParams &p = gm->prm;
     p.M = M; p.N = N; p.K = K;
-    // K bytes per k-block.  Implicit convolutions bring theirs (the channel chunk); plain GEMMs with a short K use 32-
-    // or 64-byte rows, so that the TMA does not spend its time zero-filling 128-byte rows that are mostly padding.
+    // K bytes per k-block: 32- or 64-byte rows for a short K, so that the TMA does not spend its time zero-filling 128-byte
+    // rows that are mostly padding.
     uint32_t span = K <= 32 ? 32u : (K <= 64 ? 64u : static_cast<uint32_t>(kBK));
     if (ctx->opt("no_narrow_span")) span = kBK;
     p.span = static_cast<int32_t>(span);
@@ -1018,11 +1018,11 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
     int32_t max_data = kMaxBN - extra;
     if (ctx->has_opt("tc_bn")) max_data = ctx->opt("tc_bn") >= 96 && ctx->opt("tc_bn") <= max_data ? (ctx->opt("tc_bn") & ~15) : max_data;   // tuning override, 96 columns at least
     p.tiles_m = (M + kBM - 1) / kBM;
-    // One k-block and many output channels (the MobileNetV2 expand layers): the layer's time is its epilogue's.  Tiles of
-    // at most 128 columns let two M tiles share an accumulator buffer and be requantised together, so that every load of
-    // a column's constants serves two outputs (28 x 28 x 32 -> 192 at 256 images: 24.2 -> 21.1 us; 14 x 14 x 96 -> 576:
-    // 21.7 -> 19.9 us; 56 x 56 x 24 -> 144 in its four-pixel packing, 576 columns: 73.8 -> 65.4 us; 384 and 960 columns:
-    // no change).  Not with the extra column of the activation sums, which would leave room for one M tile only.
+    // One k-block and many output channels (the MobileNetV2 expand layers): tiles of at most 128 columns, two M tiles per work unit.  At
+    // 256 images, with the rule / without (option no_narrow_n), us: 56 x 56 x 24 -> 144, whose pixel pairs are 288 columns in any case,
+    // 53.6 / 73.8; 14 x 14 x 64 -> 384 and 7 x 7 x 160 -> 960 no difference; 28 x 28 x 32 -> 192 20.1 / 17.2 and 14 x 14 x 96 -> 576
+    // 17.7 / 14.6: there the rule, made for an epilogue that loaded a column's constants once per M tile, costs.  Not with the extra
+    // column of the activation sums, which would leave room for one M tile only.
     if (!ctx->has_opt("tc_bn") && !ctx->opt("no_narrow_n") && K <= static_cast<int32_t>(span) && N > 128 && extra == 0 &&
         M > kGemvMaxM && max_data > 128)
         max_data = 128;
@@ -1126,7 +1126,7 @@ int32_t build_gemm(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &qh
         return ENN_B200_CUDA_FAILURE;
     }
     // Several small k-blocks share a pipeline stage so that a barrier round trip covers ~32 KB of operands.
-    // Implicit convolutions and narrow pointwise layers are bound by the producer's copy issue (a thread issues one tensor
+    // Narrow pointwise layers are bound by the producer's copy issue (a thread issues one tensor
     // copy per ~420 cycles and a tile needs one A and one B copy per k-block): when the weights of the only N tile fit,
     // they are loaded once per CTA and stay resident, the stages hold A only, and the producer issues half as many copies.
     const size_t b_tile = (static_cast<size_t>(p.bn_rows) * span + 1023) & ~static_cast<size_t>(1023);
@@ -1481,7 +1481,7 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
     int32_t st = ENN_B200_SUCCESS;
 
     // A GEMM whose A operand is gathered into scratch first (im2col_kernel): what the gather convolution does not cover, i.e.
-    // channel counts that are no multiple of 4.  `weight(n, k)` uses k = tap * cin + c.
+    // channel counts that are no multiple of 4 (and reductions of more than 2^20 bytes).  `weight(n, k)` uses k = tap * cin + c.
     auto make_conv_gemm = [&](TcGemm &gm, const Im2colGeom &ig, auto weight) -> int32_t {
         const int32_t K = ig.kh * ig.kw * cin;
         const int64_t M64 = static_cast<int64_t>(ig.n) * ig.oh * ig.ow;
@@ -1556,8 +1556,8 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         // f * K bytes can, which removes the gather pass; several N tiles are accepted in that case.
         int32_t pack = 1;
         // Not for layers with 96 or more output channels whose rows can be read in place: their time is the epilogue's, not
-        // the row fetches', and unpacked they keep two M tiles per work unit, which halves the epilogue's loads of the
-        // column constants (112 x 112 x 16 -> 96: 161 us packed, 152 us in place).
+        // the row fetches', and unpacked they keep two M tiles per work unit (256 images, in place / packed, us: 112 x 112 x 16 -> 96
+        // 128.2 / 145.8, 56 x 56 x 32 -> 128 42.7 / 44.6, 28 x 28 x 64 -> 128 14.1 / 15.5; packed and in 256-column tiles 112.3, 39.4 and 13.9).
         const bool epilogue_heavy = N >= 96 && (K & 15) == 0;
         if (pointwise && M64 >= 4096 && K <= 64 && !epilogue_heavy && !ctx->opt("no_pack")) {
             const int32_t zw_eff = g.w_signed ? g.w_zp : g.w_zp - 128;
@@ -1567,7 +1567,7 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
             }
             // Rows that cannot be read in place (K = 24) and whose packed form needs several N tiles anyway: the smallest
             // packing, so that an M tile's rows are copied for as few N tiles as possible (56 x 56 x 24 -> 144 at 256
-            // images: 61.5 us as pixel pairs, 65.0 us as groups of four).
+            // images: 53.6 us as pixel pairs, 58.0 us as groups of four).
             for (int32_t f = 2; f <= 8 && pack == 1 && (K & 15) != 0; f <<= 1)
                 if (f * K <= 128 && (f * K) % 16 == 0 && M64 % f == 0) pack = f;
             if (pack > 1) in_place = true;
@@ -1979,7 +1979,7 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
         ctx->last_error = buf;
         return ENN_B200_INVALID_PARAMS;
     }
-    if (!plan->gcs.empty()) {      // gathers into shared memory: no scratch array needed
+    if (!plan->gcs.empty()) {      // gathers into shared memory: no array needed
         if (*plan->err_host == 0) return gconv_execute(op, plan, in, out, nullptr, false);
         ctx->last_error = "gather convolution gave up on a barrier wait earlier";
         return ENN_B200_CUDA_FAILURE;
@@ -2046,10 +2046,12 @@ int32_t tc_execute_static(enn_b200_op *op, const void *in, void *out) {
 // placed in a 32 MiB array that belongs to the library image, so the call performs no cudaMalloc / cudaFree and no
 // allocating library routine.  The first call on a device looks the array's device address up
 // (cudaGetSymbolAddress) and encodes one tensor map; make that first call before any stream capture starts.
+// Layers that the gather convolution takes need no matrix at all; they run as by enn_b200_op_execute, from parameters of the call's own.
+// Whether a call is accepted does not depend on which kernel a layer gets: the 32 MiB limit applies to the matrix it would have.
 // Every call on a device uses the same array and leaves its last gathered matrix there; the gather overwrites all
 // the bytes the GEMM will read, so nothing needs clearing, but two calls whose kernels overlap on the GPU (different
-// streams or contexts) race on it.  Operators that need more than 32 MiB of scratch, or none, are rejected with
-// ENN_B200_INVALID_PARAMS and a message.
+// streams or contexts) race on it.  Operators whose matrix would be larger than 32 MiB, and those that read their input in
+// place, are rejected with ENN_B200_INVALID_PARAMS and a message.
 extern "C" int32_t enn_b200_op_execute_noalloc(enn_b200_op *op, const void *in_dev, void *out_dev) {
     if (!op) return ENN_B200_INVALID_PARAMS;
     if (!in_dev || !out_dev) {

@@ -59,7 +59,7 @@ CONV_CASES = {
     "signed_act": dict(n=1, h=8, w=8, cin=8, cout=8, k=3, act_dtype=cases.enn.S8, in_zp=-3, out_zp=5, per_channel=True, out_scale=0.2),
     "big_multiplier": dict(n=1, h=6, w=6, cin=4, cout=4, k=1, in_scale=0.5, w_scale=0.5, out_scale=0.05, w_zp=3),
     "batch_stem_like": dict(n=2, h=32, w=32, cin=3, cout=32, k=3, stride=2, per_channel=True, out_scale=0.1),
-    # implicit (tap-box) convolutions: swizzle spans 128 / 64 / 32, ragged grids, dilation, zero and non-zero input zero point
+    # stride-1 convolutions over multiples of 32 channels: ragged grids, dilation, zero and non-zero input zero point
     "implicit_c128": dict(n=2, h=20, w=17, cin=128, cout=48, k=3),
     "implicit_c64_56": dict(n=2, h=56, w=56, cin=64, cout=64, k=3),
     "implicit_c32_dil": dict(n=1, h=19, w=23, cin=32, cout=16, k=3, dil=2),
@@ -373,6 +373,10 @@ DECONV_CASES = {
     "implicit_c64_s3": dict(n=1, h=6, w=6, cin=64, cout=16, k=4, stride=3, pad=1),
     "s8_none_implicit": dict(n=2, h=8, w=8, cin=32, cout=16, per_channel=True, out_scale=1.2, act_dtype=cases.enn.S8, in_zp=-4, out_zp=-6),
     "s8_relu_zpm128_u8w": dict(n=1, h=7, w=9, cin=16, cout=24, act_dtype=cases.enn.S8, in_zp=3, out_zp=-128, act=cases.enn.ACT_RELU, out_scale=0.1),
+    # channel counts the gather kernel does not take: a gathered matrix and a GEMM per parity class
+    "c3": dict(n=2, h=9, w=7, cin=3, cout=20),
+    "c6_s3_pc": dict(n=1, h=8, w=9, cin=6, cout=17, k=4, stride=3, pad=1, per_channel=True, out_scale=0.3),
+    "c10_s4": dict(n=1, h=5, w=6, cin=10, cout=16, k=8, stride=4, pad=2),
 }
 
 
@@ -913,8 +917,8 @@ def test_oplist_mobilenet_small(enn, orc, ctx):
 
 
 def test_oplist_with_deconvolution(enn, orc, ctx):
-    """conv -> transposed conv -> conv in one operator list: the deconvolution's parity-class launches fork onto side
-    streams inside the captured graph and join again; results equal the oracle chain, twice (graph replay)."""
+    """conv -> transposed conv -> conv in one operator list: the deconvolution's parity classes are units of one
+    launch of the captured graph; results equal the oracle chain, twice (graph replay)."""
     d1, x, w1, b1, s1 = cases.conv_case(seed=21, n=2, h=12, w=12, cin=16, cout=32, k=3, per_channel=True, out_scale=0.2)
     y1 = orc.conv2d(d1, x, w1, b1, s1)
     d2, _, w2, b2, s2 = cases.deconv_case(seed=22, n=2, h=12, w=12, cin=32, cout=16, in_zp=int(d1.out_zp), in_scale=float(d1.out_scale))
@@ -1365,6 +1369,27 @@ def test_gather_convolution(enn, orc, ctx, name):
         _check(op, y_ref, x)
     finally:
         op.release()
+
+
+@pytest.mark.parametrize("name", ["conv:gather_s2", "g16_resident_tail_k", "g16_many_columns", "g8_k_tail", "g8_pointwise_s8", "g4_5x5_odd_n", "deconv_g8_four_classes",
+                                  "deconv_g4_stride3", "deconv_g16_staged", "deconv_taps_missing"])
+def test_gathered_matrix(enn, orc, name):
+    """The same layers through the gathered matrix (16-, 8- and 4-byte im2col) and, for transposed ones, a GEMM per parity class."""
+    if name == "conv:gather_s2":
+        kind, kw = "conv", dict(n=2, h=15, w=14, cin=32, cout=24, k=3, stride=2, w_zp=125, out_scale=0.05)
+    else:
+        kind, kw = GCONV_CASES[name]
+    case, ref, make = (cases.conv_case, orc.conv2d, enn.conv2d) if kind == "conv" else (cases.deconv_case, orc.deconv, enn.deconv)
+    d, x, w, b, sc = case(seed=_seed("matrix_" + name), **kw)
+    c = enn.Context(0)
+    try:
+        c.set_option("no_gconv", 1)
+        op = make(c, d, w, b, sc)
+        assert op.info.impl == enn.IMPL_TCGEN05 and op.info.kernel_launches == 2 * (1 if kind == "conv" else d.stride_h * d.stride_w)
+        _check(op, ref(d, x, w, b, sc), x)
+        op.release()
+    finally:
+        c.close()
 
 
 @pytest.mark.parametrize("name", ["g16_resident_tail_k", "g16_staged_wide", "g8_k_tail", "g4_5x5_odd_n", "deconv_g8_four_classes", "deconv_g16_staged", "g16_table_in_global"])

@@ -2,7 +2,7 @@
 
 Some hosts of this library may not allocate device memory once they are running (a latency-critical loop, or a
 process that handed all device memory to another component).  For them the gathered-input convolutions can keep
-their scratch matrix in a fixed array inside the library.  This file is collected last on purpose: if it fails,
+their scratch matrix, where they have one, in a fixed array inside the library.  This file is collected last on purpose: if it fails,
 a run that stops at the first failure has already executed every other test.
 """
 import ctypes as C
@@ -27,9 +27,11 @@ def _run_noalloc(enn, ctx, op, x):
 
 
 @pytest.mark.parametrize("kind,kw", [
-    ("conv", dict(n=2, h=20, w=20, cin=16, cout=32, k=3)),                                  # vector gather
+    ("conv", dict(n=2, h=20, w=20, cin=16, cout=32, k=3)),                                  # gathered inside the kernel: no array
     ("conv", dict(n=2, h=33, w=31, cin=3, cout=32, k=3, stride=2, per_channel=True, out_scale=0.1)),   # byte gather (stem-like)
-    ("deconv", dict(n=1, h=12, w=12, cin=16, cout=16)),                                     # four parity classes share the array
+    ("deconv", dict(n=1, h=12, w=12, cin=16, cout=16)),                                     # the same, four parity classes
+    ("conv", dict(n=2, h=19, w=18, cin=6, cout=32, k=3)),                                   # byte gather into the array
+    ("deconv", dict(n=1, h=12, w=11, cin=6, cout=16)),                                      # four parity classes share the array
 ])
 def test_noalloc_matches_regular_entry_point_twice(enn, ctx, kind, kw):
     if kind == "conv":
