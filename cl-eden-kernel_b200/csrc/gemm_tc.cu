@@ -1633,72 +1633,52 @@ int32_t tc_plan_conv(enn_b200_op *op, const void *w_hwio) {
         // (oy + pad_t) % sh == py only ever meet kernel rows ky = py + sh * jy, so each class (py, px) is a
         // stride-1 correlation over the input with its own small filter:
         //   out[n, sh*q - pad_t + py, ...] = sum_{jy,jx,c} in[n, q - jy, r - jx, c] * w[c][co][py + sh*jy][px + sw*jx].
-        if (!ctx->opt("no_gconv")) {
-            struct Cls { int32_t py, px, jx_e; bool empty; };
-            std::vector<GcClassDesc> cds;
-            std::vector<Cls> info;
-            for (int32_t py = 0; py < g.sh; ++py)
-                for (int32_t px = 0; px < g.sw; ++px) {
-                    const int32_t jy_n = py < g.kh ? (g.kh - py + g.sh - 1) / g.sh : 0, jx_n = px < g.kw ? (g.kw - px + g.sw - 1) / g.sw : 0;
-                    const int32_t q_lo = (g.pt - py + g.sh - 1 >= 0) ? (g.pt - py + g.sh - 1) / g.sh : 0;
-                    const int32_t q_hi = (g.oh - 1 + g.pt - py) >= 0 ? (g.oh - 1 + g.pt - py) / g.sh : -1;
-                    const int32_t r_lo = (g.pl - px + g.sw - 1 >= 0) ? (g.pl - px + g.sw - 1) / g.sw : 0;
-                    const int32_t r_hi = (g.ow - 1 + g.pl - px) >= 0 ? (g.ow - 1 + g.pl - px) / g.sw : -1;
-                    if (q_hi < q_lo || r_hi < r_lo) continue;
-                    const bool empty = jy_n == 0 || jx_n == 0;      // outputs without taps: one zero-weight dummy tap
-                    const int32_t oy0 = g.sh * q_lo - g.pt + py, ox0 = g.sw * r_lo - g.pl + px;
-                    cds.push_back({q_hi - q_lo + 1, r_hi - r_lo + 1, jy_n > 0 ? jy_n : 1, jx_n > 0 ? jx_n : 1, -1, -1, q_lo, r_lo,
-                                   (static_cast<int64_t>(oy0) * g.ow + ox0) * N});
-                    info.push_back({py, px, jx_n > 0 ? jx_n : 1, empty});
-                }
-            st = try_gconv(cds, 1, 1, static_cast<int64_t>(g.oh) * g.ow * N, static_cast<int64_t>(g.sh) * g.ow * N, static_cast<int64_t>(g.sw) * N,
-                           [&](int32_t i, int32_t n, int32_t k) -> uint8_t {
-                               const Cls &ci = info[static_cast<size_t>(i)];
-                               if (ci.empty) return static_cast<uint8_t>(g.w_zp);
-                               const int32_t tap = k / cin, c = k - tap * cin, jy = tap / ci.jx_e, jx = tap - jy * ci.jx_e;
-                               const int32_t ky = ci.py + g.sh * jy, kx = ci.px + g.sw * jx;
-                               return w[((static_cast<size_t>(ky) * g.kw + kx) * cin + c) * N + n];
-                           });
-            if (st != ENN_B200_INVALID_PARAMS) return st;
-        }
-        plan->gemms.reserve(static_cast<size_t>(g.sh) * g.sw);
-        for (int32_t py = 0; py < g.sh; ++py) {
+        struct Cls { int32_t py, px, jx_e; bool empty; };
+        std::vector<GcClassDesc> cds;
+        std::vector<Cls> info;
+        for (int32_t py = 0; py < g.sh; ++py)
             for (int32_t px = 0; px < g.sw; ++px) {
-                const int32_t jy_n = py < g.kh ? (g.kh - py + g.sh - 1) / g.sh : 0;
-                const int32_t jx_n = px < g.kw ? (g.kw - px + g.sw - 1) / g.sw : 0;
+                const int32_t jy_n = py < g.kh ? (g.kh - py + g.sh - 1) / g.sh : 0, jx_n = px < g.kw ? (g.kw - px + g.sw - 1) / g.sw : 0;
                 // q range: 0 <= sh*q - pad_t + py < oh
                 const int32_t q_lo = (g.pt - py + g.sh - 1 >= 0) ? (g.pt - py + g.sh - 1) / g.sh : 0;
                 const int32_t q_hi = (g.oh - 1 + g.pt - py) >= 0 ? (g.oh - 1 + g.pt - py) / g.sh : -1;
                 const int32_t r_lo = (g.pl - px + g.sw - 1 >= 0) ? (g.pl - px + g.sw - 1) / g.sw : 0;
                 const int32_t r_hi = (g.ow - 1 + g.pl - px) >= 0 ? (g.ow - 1 + g.pl - px) / g.sw : -1;
-                const int32_t qh_n = q_hi - q_lo + 1, qw_n = r_hi - r_lo + 1;
-                if (qh_n <= 0 || qw_n <= 0) continue;
-                // A class without taps (stride larger than the kernel) still has outputs: requant(bias).  One
-                // zero-weight dummy tap keeps it on the same code path.
-                const int32_t jy_e = jy_n > 0 ? jy_n : 1, jx_e = jx_n > 0 ? jx_n : 1;
+                if (q_hi < q_lo || r_hi < r_lo) continue;
+                // A class without taps (stride larger than the kernel) still has outputs: requant(bias).  One zero-weight dummy tap
+                // keeps it on the same code path.
                 const bool empty = jy_n == 0 || jx_n == 0;
-                plan->gemms.emplace_back();
-                TcGemm &gm = plan->gemms.back();
-                Im2colGeom ig{};
-                ig.n = g.n; ig.h = g.h; ig.w = g.w; ig.cin = cin;
-                ig.oh = qh_n; ig.ow = qw_n; ig.kh = jy_e; ig.kw = jx_e;
-                ig.sy = 1; ig.sx = 1; ig.dy = -1; ig.dx = -1; ig.y0 = q_lo; ig.x0 = r_lo;
-                ig.fill = fill;
-                st = make_conv_gemm(gm, ig, [&](int32_t n, int32_t k) -> uint8_t {
-                    const int32_t tap = k / cin, c = k - tap * cin;
-                    const int32_t jy = tap / jx_e, jx = tap - jy * jx_e;
-                    if (empty) return static_cast<uint8_t>(g.w_zp);
-                    const int32_t ky = py + g.sh * jy, kx = px + g.sw * jx;
-                    return w[((static_cast<size_t>(ky) * g.kw + kx) * cin + c) * N + n];
-                });
-                if (st != ENN_B200_SUCCESS) return bail(st);
-                gm.prm.qh = qh_n; gm.prm.qw = qw_n;
                 const int32_t oy0 = g.sh * q_lo - g.pt + py, ox0 = g.sw * r_lo - g.pl + px;
-                gm.prm.out_base = (static_cast<int64_t>(oy0) * g.ow + ox0) * N;
-                gm.prm.out_sn = static_cast<int64_t>(g.oh) * g.ow * N;
-                gm.prm.out_sy = static_cast<int64_t>(g.sh) * g.ow * N;
-                gm.prm.out_sx = static_cast<int64_t>(g.sw) * N;
+                cds.push_back({q_hi - q_lo + 1, r_hi - r_lo + 1, jy_n > 0 ? jy_n : 1, jx_n > 0 ? jx_n : 1, -1, -1, q_lo, r_lo,
+                               (static_cast<int64_t>(oy0) * g.ow + ox0) * N});
+                info.push_back({py, px, jx_n > 0 ? jx_n : 1, empty});
             }
+        const int64_t sn = static_cast<int64_t>(g.oh) * g.ow * N, s_y = static_cast<int64_t>(g.sh) * g.ow * N, s_x = static_cast<int64_t>(g.sw) * N;
+        auto class_weight = [&](int32_t i, int32_t n, int32_t k) -> uint8_t {
+            const Cls &ci = info[static_cast<size_t>(i)];
+            if (ci.empty) return static_cast<uint8_t>(g.w_zp);
+            const int32_t tap = k / cin, c = k - tap * cin, jy = tap / ci.jx_e, jx = tap - jy * ci.jx_e;
+            const int32_t ky = ci.py + g.sh * jy, kx = ci.px + g.sw * jx;
+            return w[((static_cast<size_t>(ky) * g.kw + kx) * cin + c) * N + n];
+        };
+        if (!ctx->opt("no_gconv")) {
+            st = try_gconv(cds, 1, 1, sn, s_y, s_x, class_weight);
+            if (st != ENN_B200_INVALID_PARAMS) return st;
+        }
+        plan->gemms.reserve(cds.size());
+        for (size_t i = 0; i < cds.size(); ++i) {       // a gathered matrix and a GEMM per class
+            const GcClassDesc &cd = cds[i];
+            plan->gemms.emplace_back();
+            TcGemm &gm = plan->gemms.back();
+            Im2colGeom ig{};
+            ig.n = g.n; ig.h = g.h; ig.w = g.w; ig.cin = cin;
+            ig.oh = cd.oh; ig.ow = cd.ow; ig.kh = cd.kh; ig.kw = cd.kw;
+            ig.sy = 1; ig.sx = 1; ig.dy = -1; ig.dx = -1; ig.y0 = cd.y0; ig.x0 = cd.x0;
+            ig.fill = fill;
+            st = make_conv_gemm(gm, ig, [&](int32_t n, int32_t k) { return class_weight(static_cast<int32_t>(i), n, k); });
+            if (st != ENN_B200_SUCCESS) return bail(st);
+            gm.prm.qh = cd.oh; gm.prm.qw = cd.ow;
+            gm.prm.out_base = cd.out_base; gm.prm.out_sn = sn; gm.prm.out_sy = s_y; gm.prm.out_sx = s_x;
         }
         if (plan->gemms.empty()) return bail(ENN_B200_INVALID_PARAMS);
     }
