@@ -868,6 +868,8 @@ def run_ours(args):
             peak = peaks["hbm_gbs"] if hbm else i8_peak
             ach = per_step / (res["ms"] * 1e-3)
             kname = {"depthwise": "dw3x3_ring_kernel", "add": "add_kernel_lut2", "avgpool": "avgpool_vec4_kernel"}.get(kind, KERNEL_OF_IMPL.get(res["impl"]))
+            if kind == "deconv" or args.workload.startswith("conv3x3"):
+                kname = "gconv_kernel"
             result = {
                 "metric": ("hbm_gbs_" if hbm else "int8_tops_") + args.workload, "value": world * per_step / (ms * 1e-3),
                 "unit": unit, "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,

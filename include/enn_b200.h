@@ -202,11 +202,11 @@ int32_t enn_b200_last_error(enn_b200_context *ctx, char *buf, size_t buf_len);
 /* cudaStream_t of the context, as void*, so a caller can order its own work against it. */
 void *enn_b200_stream(enn_b200_context *ctx);
 /* Planner overrides for tests and tuning, read when an operator is prepared (the library reads no environment
- * variable).  Names: no_pdl, no_relu_mode, no_relu_hi, no_relu_sat, no_wide_store, no_grouped_tc, no_first_layer, no_implicit, no_gemv, no_narrow_span, no_pack,
- * pack_wide, no_bres, no_bres_k1, no_fan_out, tc_bn (>= 96), tc_pair, tc_raster, epi_g, dw_legacy, dw_rows, no_fuse, fuse_all, no_out_stream, no_narrow_n, no_gconv,
- * gc_per_sm (1 or 2).
- * grid_cap = G: operators prepared afterwards launch at most G CTAs of their persistent kernels (tensor-core GEMM /
- * convolution, row-ring depthwise), i.e. occupy at most G SMs.  Meant for several contexts that share one GPU, each
+ * variable).  Names: no_pdl, no_relu_mode, no_relu_hi, no_relu_sat, no_grouped_tc, no_first_layer, no_gemv, no_narrow_span, no_pack,
+ * pack_wide, no_bres, no_bres_k1, tc_bn (>= 96), tc_pair, tc_raster, dw_legacy, dw_rows, no_fuse, fuse_all, no_out_stream, no_narrow_n, no_gconv,
+ * gc_per_sm (1 or 2); no_wide_store, no_implicit, no_fan_out and epi_g are accepted and change nothing.
+ * grid_cap = G: operators prepared afterwards launch at most G CTAs of their persistent tensor-core kernels (GEMM and gather
+ * convolution) and as many of the row-ring depthwise kernel as G SMs hold.  Meant for several contexts that share one GPU, each
  * running its own operator list: with G = SMs / 4 their kernels run side by side in four shares instead of taking
  * the whole GPU in turn, which hides the latency of the small layers (MobileNetV2-u8, 256 images: 1.25 ms per step
  * with eight lists of 37 SMs against 1.43 ms with three uncapped lists; 32 images: 0.22 against 0.34 ms).
@@ -278,11 +278,13 @@ int32_t enn_b200_op_fuse_add(enn_b200_op *conv, enn_b200_op *add, int32_t conv_i
  * whose tensor is not flagged is ignored (may be NULL).  Such operators cannot be added to an operator list, whose
  * captured launch sequence holds the constants' addresses. */
 int32_t enn_b200_op_rebind_constants(enn_b200_op *op, const void *weights_dev, const int32_t *bias_dev);
-/* No counterpart in the reference.  Runs a prepared Conv2D / Deconvolution whose input is gathered into a scratch
- * matrix without allocating anything: the matrix goes into a 32 MiB device array that is part of the library image.
- * For callers that may not call cudaMalloc at run time.  Limits: the operator must be on the tensor-core path and
- * need between 1 byte and 32 MiB of scratch (INVALID_PARAMS otherwise); calls that overlap on one GPU race on the
- * shared array; the first call per device does a one-time address lookup and should precede any stream capture. */
+/* No counterpart in the reference.  Runs a prepared Conv2D / Deconvolution whose input is gathered without allocating
+ * anything: where the gathered matrix is written to memory it goes into a 32 MiB device array that is part of the
+ * library image (Cin % 4 == 0: it is not written at all).  For callers that may not call cudaMalloc at run time.
+ * Limits: the operator must be on the tensor-core path, not read its input in place, and its matrix, written or not,
+ * must be at most 32 MiB (INVALID_PARAMS otherwise); calls that overlap on one GPU race on the shared array; the first
+ * call per device does a one-time address lookup and should precede any stream capture.  An armed self-test
+ * (enn_b200_op_test_starve_next) waits for enn_b200_op_execute. */
 int32_t enn_b200_op_execute_noalloc(enn_b200_op *op, const void *in_dev, void *out_dev);
 int32_t enn_b200_op_info(const enn_b200_op *op, enn_b200_op_info_t *info);
 /* Failure handling (Common.hpp:113-119 CL_FAILURE; the reference has no device-side waits to bound).  A kernel whose
