@@ -154,7 +154,8 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                 const uint32_t oy = c.div_ow.div(rem), ox = rem - oy * static_cast<uint32_t>(c.ow);
                 iy = static_cast<int>(oy) * p.sy + c.y0;
                 ix = static_cast<int>(ox) * p.sx + c.x0;
-                row += ((static_cast<int64_t>(img) * p.h + iy) * p.w + ix) * p.cin;
+                const int pixel = (static_cast<int>(img) * p.h + iy) * p.w + ix;     // fits (build_gconv)
+                row += static_cast<int64_t>(pixel) * p.cin;
             }
             asm volatile("st.shared.b64 [%0], %1;\n\tst.shared.v2.b32 [%0 + 8], {%2, %3};" ::"r"(rt + lane * 16), "l"(row), "r"(iy), "r"(ix) : "memory");
         }

@@ -1183,6 +1183,9 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
         if (M <= 0 || M > INT32_MAX - kBM || K > (1 << 20)) return ENN_B200_INVALID_PARAMS;
         // a tap's displacement is kept in 16 bits; the image itself may be of any size
         if (static_cast<int64_t>(d.kh - 1) * std::abs(d.dy) >= 32000 || static_cast<int64_t>(d.kw - 1) * std::abs(d.dx) >= 32000) return ENN_B200_INVALID_PARAMS;
+        // positions of the first tap, borders included, in pixels: 32 bits (8 GiB of 4-byte pixels, 64 GiB of 32-byte ones)
+        const int64_t last_y = static_cast<int64_t>(g.n - 1) * g.h + static_cast<int64_t>(d.oh - 1) * sy + d.y0, last_x = static_cast<int64_t>(d.ow - 1) * sx + d.x0;
+        if ((std::max<int64_t>(last_y, 0) + std::abs(d.y0)) * g.w + std::max<int64_t>(last_x, 0) + std::abs(d.x0) > INT32_MAX) return ENN_B200_INVALID_PARAMS;
         GcClass &c = p.cls[i];
         c.M = static_cast<int32_t>(M);
         c.tiles_m = static_cast<int32_t>((M + kBM - 1) / kBM);
@@ -1220,10 +1223,11 @@ int32_t build_gconv(enn_b200_context *ctx, const ConvGeom &g, const QuantHost &q
     // 1.25 + 0.95 * columns / 256 rounds of single units (64 columns 1.46, 128 1.70, 176 1.9, 256 2.2), so whole rounds decide.  us
     // with two / with one, 3x3: 128x14x14x512 -> 512 71 / 47, 16x56x56x256 -> 256 40.7 / 28.1, 64x28x28x96 -> 192 17.9 / 13.8;
     // 32x56x56x128 -> 128 22.0 / 25.8, 256x56x56x64 -> 64 70.9 / 94.8.  Not for 8- and 4-byte gathers (158x27x27x72 -> 184 38.1 / 39.7) and
-    // reductions of one or two k-blocks, whose time is the epilogue's.
+    // reductions of one or two k-blocks, whose time is the epilogue's; for three and four by a margin (15x38x38x32 -> 224 7.3 / 7.5).
     {
         const int64_t single = (p.n_units + sms - 1) / sms, pairs = (p.n_units + 2 * sms - 1) / (2 * sms);
-        const bool alone = p.n_units > sms && p.unit == 16 && kb_total > 2 * nc && single * 256 * 100 < pairs * (125 * 256 + 95 * p.bn_rows);
+        const int64_t margin = kb_total > 4 * nc ? 100 : 105;
+        const bool alone = p.n_units > sms && p.unit == 16 && kb_total > 2 * nc && single * 256 * margin < pairs * (125 * 256 + 95 * p.bn_rows);
         // A share of the SMs (option grid_cap) is that many CTAs, of which each may have an SM for itself.
         if (sms < ctx->sm_count) gc->per_sm = 1;
         else gc->per_sm = ctx->has_opt("gc_per_sm") ? (ctx->opt("gc_per_sm") == 1 ? 1 : 2) : (alone ? 1 : 2);
