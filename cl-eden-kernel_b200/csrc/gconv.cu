@@ -157,7 +157,8 @@ __device__ __forceinline__ void gather_role(const GcParams &p, const GcSmem &L, 
                 const int pixel = (static_cast<int>(img) * p.h + iy) * p.w + ix;     // fits (build_gconv)
                 row += static_cast<int64_t>(pixel) * p.cin;
             }
-            asm volatile("st.shared.b64 [%0], %1;\n\tst.shared.v2.b32 [%0 + 8], {%2, %3};" ::"r"(rt + lane * 16), "l"(row), "r"(iy), "r"(ix) : "memory");
+            const uint64_t addr = reinterpret_cast<uint64_t>(row);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rt + lane * 16), "r"(static_cast<uint32_t>(addr)), "r"(static_cast<uint32_t>(addr >> 32)), "r"(iy), "r"(ix) : "memory");
         }
         __syncwarp();
         if (!waited) {
